@@ -151,7 +151,7 @@ int ensure_ready(int dev, DeviceInfo** out) {
     S.info.cc_minor = p.minor;
     S.info.total_mem = p.totalGlobalMem;
     if (!tk::mma_init_device(&S.info) || !tk::matvec_init_device() ||
-        !tk::tc5_init_device(&S.info)) {
+        !tk::tc5_init_device(&S.info) || !tk::pack_init_device(&S.info)) {
       set_err("kernel set-up", cudaGetLastError());
       return TK_ERR_CUDA;
     }

@@ -82,6 +82,12 @@ bool tc5_init_device(DeviceInfo* info);
 cudaError_t launch_tc5(bool inverse, const int16_t* src, int16_t* dst, long long npoly,
                        const DeviceInfo& info, cudaStream_t stream);
 
+// The dense packed forward (tk_pack.cu), bits = 2 or 3; npoly at most
+// kMaxLaunchPolys.
+bool pack_init_device(DeviceInfo* info);
+cudaError_t launch_packed(int bits, const void* src, int16_t* dst, int npoly,
+                          const DeviceInfo& info, cudaStream_t stream);
+
 // Matrix-vector jobs (tk_matvec.cu).  Chunks hold at most this many vector
 // polynomials, so that intermediates stay in the 126 MB L2.
 constexpr long long kMatvecChunkVecPolys = 131072;  // default (64 MiB); tk_set_option may change it

@@ -1172,6 +1172,13 @@ static cudaError_t launch_variant(const Variant& V, long long cap, const P& m, l
   return cudaLaunchKernelExC(&cfg, V.fn, args);
 }
 
+// Packed inputs above two full waves of the mma.sync form's 32-polynomial tiles
+// (28,416 polynomials on 148 SMs) run the dense kernel (tk_pack.cu).  Below,
+// its 128-polynomial tiles leave SMs idle and its longer chain per tile shows:
+// 2-bit, us, mma.sync / dense: 4,096 2.9 / 5.4, 12,000 4.3 / 5.7, 20,011 6.4 /
+// 7.0; above: 32,768 9.4 / 7.5, 100,003 21.7 / 16.0, 262,144 50.1 / 30.0, 2^20
+// 187.1 / 104.7 (3-bit 191.4 / 114.3).
+
 cudaError_t launch_fwd_form(int form, const void* src, int16_t* dst, long long npoly,
                             const DeviceInfo& info, cudaStream_t stream) {
   if (form < 1 || form > kNumInputForms) return cudaErrorInvalidValue;
@@ -1181,6 +1188,11 @@ cudaError_t launch_fwd_form(int form, const void* src, int16_t* dst, long long n
   for (long long done = 0; done < npoly; done += kMaxLaunchPolys) {
     const int n = (int)((npoly - done) < kMaxLaunchPolys ? (npoly - done) : kMaxLaunchPolys);
     const uint8_t* in = (const uint8_t*)src + done * row_bytes;
+    if (form != kInSmall && n > 2 * cap * V.tile) {
+      const cudaError_t e = launch_packed(form, in, dst + done * 256, n, info, stream);
+      if (e != cudaSuccess) return e;
+      continue;
+    }
     OneSeg m = {};
     const bool ok_in = form == kInSmall ? encode_batch_map(&m.in, (const int16_t*)in, n)
                                         : encode_packed_map(&m.in, in, n, row_bytes);

@@ -284,4 +284,25 @@ void build_tc5_tables(const Matrices& M, uint8_t* out) {
         }
 }
 
+void build_pack_tables(int bits, uint8_t* out) {
+  const int s = 8 - bits;
+  int64_t v[256];
+  int16_t F[128][128];
+  for (int j = 0; j < 128; j++) {
+    memset(v, 0, sizeof(v));
+    v[2 * j] = 1;
+    fwd_layers(v, 128, 2);
+    for (int t = 0; t < 128; t++)
+      F[t][j] = (int16_t)(v[2 * t] > (kQ - 1) / 2 ? v[2 * t] - kQ : v[2 * t]);
+  }
+  for (int t = 0; t < 128; t++)
+    for (int k = 0; k < 256; k++) {
+      const PackPos at = pack_k_pos(bits, k);
+      const int c = F[t][at.j], half = 1 << (s - 1);
+      const int c0 = ((c + half) & ((1 << s) - 1)) - half, c1 = (c - c0) >> s;
+      out[2048 * (8 * (t >> 6) + (k >> 5)) + tc5_tile_offset(t & 63, k & 31)] =
+          (uint8_t)(int8_t)(at.top ? c1 : c0);
+    }
+}
+
 }  // namespace tk

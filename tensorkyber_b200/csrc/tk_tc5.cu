@@ -67,6 +67,7 @@
 #include "tk_internal.h"
 #include "tk_ptx.cuh"
 #include "tk_tables.h"
+#include "tk_umma.cuh"
 
 namespace tk {
 namespace {
@@ -109,11 +110,9 @@ struct Tc5Layout {
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColY = 0;
 constexpr uint32_t kColD0 = 256;  // group g's accumulator buffer at kColD0 + 64 g
-// instruction descriptors of kind::i8: D format s32 (bits 4-5 = 2), A / B
-// format (bits 7-9 / 10-12: 0 unsigned, 1 signed), K-major A and B, N >> 3
-// (bits 17-22) = 4, M >> 4 (bits 24-28) = 8: M = 128, N = 32, K = 32.
-constexpr uint32_t kIdescU8 = (2u << 4) | (4u << 17) | (8u << 24);
-constexpr uint32_t kIdescS8 = kIdescU8 | (1u << 7) | (1u << 10);
+// instruction descriptors: M = 128, N = 32, K = 32, both operands of one type
+constexpr uint32_t kIdescU8 = idesc_i8(32, false, false);
+constexpr uint32_t kIdescS8 = idesc_i8(32, true, true);
 constexpr uint64_t kWaitNs = 2000000000ull;
 // The first stage's sums S (in [-16 * 128 (q-1), 16 * 382 (q-1)]: unsigned
 // low bytes and signed high bytes against constants below q) plus this
@@ -123,32 +122,6 @@ constexpr uint32_t kFirstBias = 2048u * 3329u;
 
 __device__ __align__(128) uint8_t g_tc5_tables[kTc5TableBytes];
 
-// Shared-memory matrix descriptor (sm_100 format: start, leading and stride
-// byte offsets in 16-byte units, version 1 at bit 46, layout at bits 61-63).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo,
-                                              uint32_t layout) {
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | ((uint64_t)layout << 61);
-}
-constexpr uint32_t kLayoutNone = 0, kLayoutSw128 = 2;
-
-__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t a) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
-}
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c,
-                                             uint32_t d) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
-               "r"(d)
-               : "memory");
-}
-__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(addr)
-               : "memory");
-  return v;
-}
 __device__ __forceinline__ uint32_t word_of(const uint4& v, int i) {
   return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
 }
@@ -568,28 +541,39 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
   return fn;
 }
 
-// The batch as a [npoly][256] uint16 tensor: boxes of 64 coefficients x 128
-// polynomials with the 128-byte swizzle (16 KiB each, four per tile).
-bool encode_swizzled_map(CUtensorMap* map, const int16_t* base, int npoly) {
+const uint8_t* g_tables_ptr[64];
+
+}  // namespace
+
+static bool encode_tile_map(CUtensorMap* map, CUtensorMapDataType type, const void* base,
+                            cuuint64_t cols, cuuint64_t row_bytes, cuuint32_t box_cols, int npoly,
+                            CUtensorMapSwizzle swizzle) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
   if (!enc) {
     note_encode_result(-1);
     return false;
   }
-  const cuuint64_t dims[2] = {256, (cuuint64_t)npoly};
-  const cuuint64_t strides[1] = {512};
-  const cuuint32_t box[2] = {64, (cuuint32_t)kTcTile};
+  const cuuint64_t dims[2] = {cols, (cuuint64_t)npoly};
+  const cuuint64_t strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {box_cols, (cuuint32_t)kTcTile};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void*)base, dims, strides, box,
-                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = enc(map, type, 2, (void*)base, dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   note_encode_result((int)r);
   return r == CUDA_SUCCESS;
 }
 
-const uint8_t* g_tables_ptr[64];
+bool encode_swizzled_map(CUtensorMap* map, const int16_t* base, int npoly) {
+  return encode_tile_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, base, 256, 512, 64, npoly,
+                         CU_TENSOR_MAP_SWIZZLE_128B);
+}
 
-}  // namespace
+bool encode_packed_tile_map(CUtensorMap* map, const void* base, int npoly, int row_bytes) {
+  return encode_tile_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, base, (cuuint64_t)row_bytes / 4,
+                         (cuuint64_t)row_bytes, (cuuint32_t)row_bytes / 4, npoly,
+                         row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+}
 
 bool tc5_init_device(DeviceInfo* info) {
   static uint8_t image[kTc5TableBytes];
