@@ -124,9 +124,11 @@ __device__ __forceinline__ void cta_sync_named() {
 
 // Block-wise stage of one tile for this warp: P block pairs x NT n-tiles of 8
 // polynomials (NT = W: a full tile), the next unit's ldmatrix issued ahead of
-// the current stores.  Inverse input is biased (x ^ 0x8000) and parity-split
-// here; forward input is already parity-split by stage 1.
-template <bool kInverse, int W, int P, int NT = W>
+// the current stores.  kSplit: the input is parity-split already (by the
+// forward's stage 1, or the tiled kernel's basemul); otherwise it is the
+// inverse's natural-order int16, biased (x ^ 0x8000) and parity-split here.
+// kLazy: the output's reduction (stage_c).
+template <bool kSplit, bool kLazy, int W, int P, int NT = W>
 __device__ __forceinline__ void block_stage(uint32_t slot, uint8_t* slotp, int blk0,
                                             uint32_t ldc_off, uint32_t stc_off,
                                             const uint32_t (&ac)[P][2][2][2],
@@ -144,7 +146,7 @@ __device__ __forceinline__ void block_stage(uint32_t slot, uint8_t* slotp, int b
               n[3]);
     }
     uint32_t x[4];
-    if (kInverse) {
+    if (!kSplit) {
       // r = (I: c 2q,2q+1 | I: c 8+2q,9+2q | I+1: ...); bias, then parity split
       // into slots (c=2q | c=8+2q) and (c=2q+1 | c=9+2q)
       const uint32_t x0 = r[0] ^ 0x80008000u, x1 = r[1] ^ 0x80008000u;
@@ -157,7 +159,7 @@ __device__ __forceinline__ void block_stage(uint32_t slot, uint8_t* slotp, int b
 #pragma unroll
       for (int j = 0; j < 4; j++) x[j] = r[j];
     }
-    stage_c<kInverse>(ac[p], cc[p], x,
+    stage_c<kLazy>(ac[p], cc[p], x,
                       slotp + nt * 8 * kRowBytes + 32 * (blk0 + 2 * p) + stc_off);
 #pragma unroll
     for (int j = 0; j < 4; j++) r[j] = n[j];
@@ -672,12 +674,12 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
         if (u_begin + k * W + warp < u_end) bad |= tile_bad;
       }
       cta_sync_named();
-      block_stage<false, W>(slot, slotp, blk0, ldc_off, stc_off, ac, cc);
+      block_stage<true, false, W>(slot, slotp, blk0, ldc_off, stc_off, ac, cc);
       fence_proxy_async_smem();
       cta_sync_named();
       issue_store(k, slot_i);
     } else {
-      block_stage<true, W>(slot, slotp, blk0, ldc_off, stc_off, ac, cc);
+      block_stage<false, true, W>(slot, slotp, blk0, ldc_off, stc_off, ac, cc);
       cta_sync_named();
       const int unit = u_begin + k * W + warp;
       const int sg = kAdd ? seg_of(unit) : 0;
@@ -721,6 +723,12 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
 // constants are re-read from L1 at each stage, so that between stages their
 // registers hold the basemul's loads in flight.  Every mbarrier wait is
 // bounded (2 s; sets status bit 4 and stops the CTA).
+// Bound by instruction issue and load latency (16 warps per SM at about half
+// the issue slots), not DRAM, so instructions come out wherever an
+// intermediate's form is this kernel's own: ntt(s) reduced lazily, A words
+// multiplied packed (dp2a), the accumulators written parity-split and unbiased
+// for stage A, e added as packed pairs.  65,536 jobs, k ~ U{2,3,4}: 143.8 ->
+// 133.3 us (4.7 TB/s of A, s, e and out); 1,023 jobs 7.8 -> 7.05 us.
 struct MvTiles {
   CUtensorMap s_map[kMaxSegs];    // s rows [njobs * k][128 words], 8 x 132-word boxes
   CUtensorMap out_map[kMaxSegs];  // out rows, the same shape (may equal s_map: in place)
@@ -733,8 +741,10 @@ struct MvTiles {
 };
 
 __device__ int32_t g_tile_z[128];  // basemul pair roots z_t (build_pair_roots)
-// The tiled kernel's inverse: g_inv with stage B scaled by 2^-16, the factor
-// its basemul leaves out (basemul_row_z).
+// The tiled kernel's inverse: stage A on the basemul's parity-split rows
+// (non-negative: no bias to cancel), stage B scaled by 2^-16, the factor its
+// basemul leaves out (basemul_row_z).
+__device__ TileFrags g_tile_sa;
 __device__ InvFrags g_tile_inv;
 
 constexpr int kTileSlotBytes = 32 * kRowBytes;      // one 32-row slot
@@ -810,9 +820,14 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   const uint32_t w_nat = 32u * g8 + 4u * q4;
   const uint32_t hbw = (uint32_t)((blk0 >> 2) & 1);
   const uint32_t ldc_base = kRowBytes * (lane & 7) + 32u * (lane >> 4);
-  const uint32_t ldc_fwd = ldc_base + 16u * (((lane >> 3) & 1) ^ hbw);
-  const uint32_t ldc_inv = ldc_base + 16u * ((lane >> 3) & 1);
+  const uint32_t ldc_split = ldc_base + 16u * (((lane >> 3) & 1) ^ hbw);
   const uint32_t stc_off = kRowBytes * (2 * q4) + 4u * g8;
+  // basemul output: lane l owns coefficients 8l .. 8l+7, half of block l / 2;
+  // its even and odd ones go to the block's parity halves, which are swapped in
+  // blocks with bit 2 set (the 8-byte stores of a half-warp then meet no bank
+  // twice), as stage A's reads (ldc_split) expect
+  const uint32_t acc_even = 32u * (lane >> 1) + 16u * ((lane >> 3) & 1) + 8u * (lane & 1);
+  const uint32_t acc_odd = acc_even ^ 16u;
   // the inverse's intermediate with block halves swapped where bit 2 of the
   // block is set (as the batch kernel's): stage A's stores, stage B's rows
   const uint32_t stc_inv = kRowBytes * (2 * q4) + 4u * (g8 ^ (4 * hbw));
@@ -867,7 +882,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     cta_sync_named();
     uint32_t fac[PP][2][2][2];
     load_ac(g_fwd.s2, fac);
-    block_stage<false, W, PP, NU>(slot, slotp, blk0, ldc_fwd, stc_off, fac, zc);
+    block_stage<true, true, W, PP, NU>(slot, slotp, blk0, ldc_split, stc_off, fac, zc);
   };
   // basemul-accumulate into the accumulator tile, one job per warp at a
   // time, all k^2 loads of A issued first
@@ -879,20 +894,23 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       const int job = tl * kJobs + jl;
       if (job >= njobs) break;  // warp-uniform
       const int16_t* Aj = P.A[b] + (size_t)job * K * K * 256 + 8 * lane;
-      uint4 a[K][K], bv[K];
-      uint2 zb[K];
+      uint4 a[K][K];
+      BasemulOperand bv[K];
 #pragma unroll
       for (int i = 0; i < K; i++)
 #pragma unroll
         for (int j = 0; j < K; j++) a[i][j] = __ldcs((const uint4*)(Aj + (i * K + j) * 256));
 #pragma unroll
-      for (int j = 0; j < K; j++) {
-        bv[j] = *(const uint4*)(slotp + (jl * K + j) * kRowBytes + 16 * lane);
-        zb[j] = pair_zb(bv[j], zt);
-      }
+      for (int j = 0; j < K; j++)
+        bv[j] = basemul_operand(*(const uint4*)(slotp + (jl * K + j) * kRowBytes + 16 * lane), zt);
 #pragma unroll
-      for (int i = 0; i < K; i++)
-        *(uint4*)(accp + (jl * K + i) * kRowBytes + 16 * lane) = basemul_row_z<K>(a[i], bv, zb);
+      for (int i = 0; i < K; i++) {
+        uint2 even, odd;
+        basemul_row_z<K>(a[i], bv, &even, &odd);
+        uint8_t* const row = accp + (jl * K + i) * kRowBytes;
+        *(uint2*)(row + acc_even) = even;
+        *(uint2*)(row + acc_odd) = odd;
+      }
     }
   };
   // inverse NTT plus e on the accumulator tile, in place; then the store
@@ -900,24 +918,16 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     constexpr int NU = decltype(nc)::value;
     {
       uint32_t iac[PP][2][2][2];
-      load_ac(g_inv.sa, iac);
-      block_stage<true, W, PP, NU>(acc, accp, blk0, ldc_inv, stc_inv, iac, zc);
+      load_ac(g_tile_sa.sa, iac);
+      block_stage<true, true, W, PP, NU>(acc, accp, blk0, ldc_split, stc_inv, iac, zc);
     }
     cta_sync_named();
     if (warp < NU) {
       uint32_t iam[2][4];
       load_am(g_tile_inv.sb, iam);
-      int32_t cb[2][4];
-#pragma unroll
-      for (int t = 0; t < 2; t++) {
-        const uint4 v = ldg_keep_u4(&g_tile_inv.cbz[lane][t][0]);
-        cb[t][0] = (int32_t)v.x;
-        cb[t][1] = (int32_t)v.y;
-        cb[t][2] = (int32_t)v.z;
-        cb[t][3] = (int32_t)v.w;
-      }
+      const int32_t cbz[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
       poly_stage<true, true>(acc + 8 * warp * kRowBytes, accp + 8 * warp * kRowBytes, ldt_inv, iam,
-                             0, 0, cb, 0, 0, w_nat, P.e[b], row0 + 8 * warp, nvec, 8u * g8 + q4);
+                             0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + 8 * warp, nvec, 8u * g8 + q4);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0 && row0 + 8 * warp < nvec)  // boxes past the batch are dropped
@@ -1070,9 +1080,11 @@ static bool upload_tables_current_device() {
   static Matrices M, MR;
   static FwdFrags FF;
   static InvFrags IF, IFR;
+  static TileFrags TF;
   static std::once_flag once;
   std::call_once(once, [] {
     build_matrices(&M);
+    build_tile_frags(M, &TF);
     build_fwd_frags(M, &FF);
     build_inv_frags(M, &IF);
     MR = M;
@@ -1082,6 +1094,7 @@ static bool upload_tables_current_device() {
   if (cudaMemcpyToSymbol(g_fwd, &FF, sizeof(FF)) != cudaSuccess) return false;
   if (cudaMemcpyToSymbol(g_inv, &IF, sizeof(IF)) != cudaSuccess) return false;
   if (cudaMemcpyToSymbol(g_tile_inv, &IFR, sizeof(IFR)) != cudaSuccess) return false;
+  if (cudaMemcpyToSymbol(g_tile_sa, &TF, sizeof(TF)) != cudaSuccess) return false;
   int32_t z[128];
   build_pair_roots(z);
   if (cudaMemcpyToSymbol(g_tile_z, z, sizeof(z)) != cudaSuccess) return false;

@@ -192,6 +192,24 @@ __device__ __forceinline__ uint32_t red_centred(uint32_t s) {
 __device__ __forceinline__ uint32_t pack2(uint32_t lo, uint32_t hi) {
   return __byte_perm(lo, hi, 0x5410);
 }
+// Two int16 additions, each wrapping.
+__device__ __forceinline__ uint32_t add16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("add.s16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+// c + a.h0 b.b0 + a.h1 b.b1 (lo) or c + a.h0 b.b2 + a.h1 b.b3 (hi): signed
+// halves of a, unsigned bytes of b.
+__device__ __forceinline__ uint32_t dp2a_lo(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("dp2a.lo.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ uint32_t dp2a_hi(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("dp2a.hi.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
 
 }  // namespace tk
 

@@ -72,20 +72,16 @@ __device__ __forceinline__ void stage_m_out(const int32_t (&lo0)[4], const int32
   }
   // D regs: [0] (row i, c=2q), [1] (row i, c=2q+1), [2]/[3] row i+8; n-tile 1 is c+8.
   if (kInverse) {  // natural order; plus the addend pairs (int16 wrap-around add)
+    uint32_t w[4] = {pack2(y0[0], y0[1]), pack2(y1[0], y1[1]), pack2(y0[2], y0[3]),
+                     pack2(y1[2], y1[3])};
     if (kAdd) {
-    y0[0] += (uint32_t)(int32_t)(int16_t)(add[0] & 0xffffu);
-    y0[1] += (uint32_t)((int32_t)add[0] >> 16);
-    y1[0] += (uint32_t)(int32_t)(int16_t)(add[1] & 0xffffu);
-    y1[1] += (uint32_t)((int32_t)add[1] >> 16);
-    y0[2] += (uint32_t)(int32_t)(int16_t)(add[2] & 0xffffu);
-    y0[3] += (uint32_t)((int32_t)add[2] >> 16);
-    y1[2] += (uint32_t)(int32_t)(int16_t)(add[3] & 0xffffu);
-    y1[3] += (uint32_t)((int32_t)add[3] >> 16);
+#pragma unroll
+      for (int j = 0; j < 4; j++) w[j] = add16x2(w[j], add[j]);
     }
-    *(uint32_t*)(row + w_nat) = pack2(y0[0], y0[1]);
-    *(uint32_t*)(row + w_nat + 16) = pack2(y1[0], y1[1]);
-    *(uint32_t*)(row + w_nat + 256) = pack2(y0[2], y0[3]);
-    *(uint32_t*)(row + w_nat + 256 + 16) = pack2(y1[2], y1[3]);
+    *(uint32_t*)(row + w_nat) = w[0];
+    *(uint32_t*)(row + w_nat + 16) = w[1];
+    *(uint32_t*)(row + w_nat + 256) = w[2];
+    *(uint32_t*)(row + w_nat + 256 + 16) = w[3];
   } else {  // parity-split slots (c=2q | c=8+2q), (c=2q+1 | c=9+2q)
     *(uint32_t*)(row + w_even) = pack2(y0[0], y1[0]);
     *(uint32_t*)(row + w_odd) = pack2(y0[1], y1[1]);
@@ -229,8 +225,9 @@ __device__ __forceinline__ uint32_t packed_operand(uint32_t w0, uint32_t w1, uin
 
 // Block-wise stage (forward stage 2 / inverse stage A) for blocks I, I+1 of 8
 // polynomials.  r[0..3]: B operands (even I, odd I, even I+1, odd I+1).
-// Output: natural order, polynomials 2q and 2q+1 of the n-tile.
-template <bool kInverse>
+// Output: natural order, polynomials 2q and 2q+1 of the n-tile; kLazy: reduced
+// to [0, q + 22) (sums below 2^26), else exactly to [0, q).
+template <bool kLazy>
 __device__ __forceinline__ void stage_c(const uint32_t (&a)[2][2][2], const int32_t (&ca)[2][2],
                                         const uint32_t (&r)[4], uint8_t* out) {
 #pragma unroll
@@ -245,7 +242,7 @@ __device__ __forceinline__ void stage_c(const uint32_t (&a)[2][2][2], const int3
     const uint32_t so0 = (uint32_t)dodd[0] + ((uint32_t)dodd[2] << 7);
     const uint32_t so1 = (uint32_t)dodd[1] + ((uint32_t)dodd[3] << 7);
     uint32_t e0, e1, o0, o1;
-    if (kInverse) {
+    if (kLazy) {
       e0 = red_lazy(se0); e1 = red_lazy(se1); o0 = red_lazy(so0); o1 = red_lazy(so1);
     } else {
       e0 = red_exact(se0); e1 = red_exact(se1); o0 = red_exact(so0); o1 = red_exact(so1);
@@ -350,43 +347,59 @@ __device__ __forceinline__ uint4 basemul_row(const uint4 (&a)[K], const uint4 (&
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// The same products with z folded into ntt(s) and 2^-16 left to the caller
-// (the tiled kernel's inverse tables carry it).  zb = the lane's z_t * b1
-// for its four pairs of one polynomial (b1 in [0, q)), as 16-bit values in
-// [0, q + 4): red_wide of a product below q^2 is off by less than 0.002 q.
-__device__ __forceinline__ uint2 pair_zb(const uint4 b, const uint32_t (&z)[4]) {
-  const uint32_t p0 = red_wide((b.x >> 16) * z[0]), p1 = red_wide((b.y >> 16) * z[1]);
-  const uint32_t p2 = red_wide((b.z >> 16) * z[2]), p3 = red_wide((b.w >> 16) * z[3]);
-  return make_uint2(p0 | (p1 << 16), p2 | (p3 << 16));
-}
-
-constexpr uint32_t kSumBiasZ = 3329u << 19;  // >= |sum| (< 2^29.71); sum + bias < 2^32
-
-// Per pair, out0 = sum_j a0 b0 + a1 (z b1), out1 = sum_j a0 b1 + a1 b0, each
-// reduced once: 2^16 times the reference's basemul-accumulate, mod q.  With
-// b0, b1 < q and z b1 < q + 4, |sum| <= 2K * 32768 * (q + 3) < 2^29.71 for
-// K <= 4, so the biased sums lie in [0, 2^32) and red_wide leaves [0, 1.41 q).
-template <int K>
-__device__ __forceinline__ uint4 basemul_row_z(const uint4 (&a)[K], const uint4 (&b)[K],
-                                               const uint2 (&zb)[K]) {
-  uint32_t o[4];
+// The same products with z folded into ntt(s), 2^-16 left to the caller (the
+// tiled kernel's inverse tables carry it) and two products per instruction:
+// dp2a multiplies the two int16 of an A word by two bytes of one ntt(s)
+// operand word, so a pair's A word is never unpacked.  Per pair and j, with
+// b0, b1 = ntt(s_j) in [0, q + 22) and zb = z_t b1 mod q in [0, q + 4)
+// (red_wide of a product below 2^24), the operand words are the bytes
+//   w0 = b0.lo, zb.lo, b0.hi, zb.hi     w1 = b1.lo, b0.lo, b1.hi, b0.hi
+// Bound by instructions and load latency: 4 dp2a per pair and j against 4
+// multiply-adds and 2 unpacks, 2 byte permutes per word pair against 3 unpacks.
+struct BasemulOperand {
+  uint32_t w0[4], w1[4];
+};
+__device__ __forceinline__ BasemulOperand basemul_operand(const uint4 b, const uint32_t (&z)[4]) {
+  BasemulOperand o;
+  const uint32_t w[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
   for (int u = 0; u < 4; u++) {
-    uint32_t t0 = kSumBiasZ, t1 = kSumBiasZ;
+    const uint32_t zb = red_wide((w[u] >> 16) * z[u]);
+    o.w0[u] = __byte_perm(w[u], zb, 0x5140);
+    o.w1[u] = __byte_perm(w[u], 0, 0x1302);
+  }
+  return o;
+}
+
+constexpr uint32_t kSumBiasZ = 3329u << 19;  // >= |sum| (< 2^29.72); sum + bias < 2^32
+
+// One lane's four output pairs of row i: out0 = sum_j a0 b0 + a1 zb, out1 =
+// sum_j a0 b1 + a1 b0, each reduced once: 2^16 times the reference's
+// basemul-accumulate, mod q.  |sum| <= 2K * 32768 * (q + 21) < 2^29.72 for K
+// <= 4, so the biased sums lie in [0, 2^32) and red_wide leaves [0, 1.41 q).
+// The pairs' even coefficients come back in `even` and the odd ones in `odd`
+// (two int16 per word, in order): the parity-split form that the tiled
+// kernel's stage A reads.
+template <int K>
+__device__ __forceinline__ void basemul_row_z(const uint4 (&a)[K], const BasemulOperand (&b)[K],
+                                              uint2* even, uint2* odd) {
+  uint32_t r0[4], r1[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    uint32_t l0 = kSumBiasZ, l1 = kSumBiasZ, h0 = 0, h1 = 0;
 #pragma unroll
     for (int j = 0; j < K; j++) {
       const uint32_t aw = u == 0 ? a[j].x : u == 1 ? a[j].y : u == 2 ? a[j].z : a[j].w;
-      const uint32_t bw = u == 0 ? b[j].x : u == 1 ? b[j].y : u == 2 ? b[j].z : b[j].w;
-      const uint32_t zw = u < 2 ? zb[j].x : zb[j].y;
-      const int32_t a0 = (int16_t)(aw & 0xffffu), a1 = (int32_t)aw >> 16;
-      const int32_t b0 = (int32_t)(bw & 0xffffu), b1 = (int32_t)(bw >> 16);
-      const int32_t z1 = (int32_t)((u & 1) ? zw >> 16 : zw & 0xffffu);
-      t0 += (uint32_t)(a0 * b0 + a1 * z1);
-      t1 += (uint32_t)(a0 * b1 + a1 * b0);
+      l0 = dp2a_lo(aw, b[j].w0[u], l0);
+      h0 = dp2a_hi(aw, b[j].w0[u], h0);
+      l1 = dp2a_lo(aw, b[j].w1[u], l1);
+      h1 = dp2a_hi(aw, b[j].w1[u], h1);
     }
-    o[u] = pack2(red_wide(t0), red_wide(t1));
+    r0[u] = red_wide(l0 + (h0 << 8));
+    r1[u] = red_wide(l1 + (h1 << 8));
   }
-  return make_uint4(o[0], o[1], o[2], o[3]);
+  *even = make_uint2(pack2(r0[0], r0[1]), pack2(r0[2], r0[3]));
+  *odd = make_uint2(pack2(r1[0], r1[1]), pack2(r1[2], r1[3]));
 }
 
 }  // namespace tk

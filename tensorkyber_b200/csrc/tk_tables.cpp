@@ -255,6 +255,16 @@ void build_inv_frags(const Matrices& M, InvFrags* F) {
     }
 }
 
+void build_tile_frags(const Matrices& M, TileFrags* F) {
+  for (int b = 0; b < 16; b++)
+    for (int s = 0; s < 2; s++)
+      pack_a_k16(
+          [&](int r, int k) {
+            return limb(byte_weighted(M.ma[b][2 * (r & 7) + s][2 * (k >> 1) + s], k & 1), r >> 3);
+          },
+          F->sa[b][s]);
+}
+
 void build_tc5_tables(const Matrices& M, uint8_t* out) {
   memset(out, 0, kTc5TableBytes);
   auto put = [&](int tile, int n, int k, int64_t v) {

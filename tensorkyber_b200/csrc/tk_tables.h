@@ -103,6 +103,13 @@ struct InvFrags {
   int32_t cbz[32][2][4];
 };
 
+// Stage A of the tiled matrix-vector kernel: as InvFrags::sa, but with slot j
+// of parity s holding coefficient c' = 2 j + s (its basemul writes each parity
+// in order) and non-negative inputs (no bias, no correction).
+struct TileFrags {
+  uint32_t sa[16][2][32][2];
+};
+
 // Logical matrices (canonical residues in [0, q)).
 struct Matrices {
   int16_t m1[16][16];        // [i][m]
@@ -177,6 +184,7 @@ void build_pack_tables(int bits, uint8_t* out /* kPackTableBytes */);
 void build_matrices(Matrices* M);
 void build_fwd_frags(const Matrices& M, FwdFrags* F);
 void build_inv_frags(const Matrices& M, InvFrags* F);
+void build_tile_frags(const Matrices& M, TileFrags* F);
 
 // Slot order inside a forward stage-2 parity half.
 inline int fwd_slot_e(int slot) { return (slot >> 1) + 4 * (slot & 1); }
