@@ -748,7 +748,7 @@ __device__ TileFrags g_tile_sa;
 __device__ InvFrags g_tile_inv;
 
 constexpr int kTileSlotBytes = 32 * kRowBytes;      // one 32-row slot
-constexpr int kTileSmem = 3 * kTileSlotBytes + 16;  // s slot x 2, accumulators, 2 mbarriers
+constexpr int kTileSmem = 2 * kTileSlotBytes + 16;  // two tile slots, 2 mbarriers
 __host__ __device__ constexpr int tile_units(int k) { return k == 3 ? 3 : 4; }
 __host__ __device__ constexpr int tile_jobs(int k) { return 8 * tile_units(k) / k; }
 
@@ -764,9 +764,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   const int G = (int)gridDim.x;
   const int nmine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / G + 1 : 0;
   const uint32_t smem0 = smem_u32(smem);
-  const uint32_t acc = smem0 + 2 * kTileSlotBytes;
-  uint8_t* const accp = smem + 2 * kTileSlotBytes;
-  const uint32_t bar0 = smem0 + 3 * kTileSlotBytes;
+  const uint32_t bar0 = smem0 + 2 * kTileSlotBytes;
 
   const int blk0 = 4 * warp;
   int32_t zc[PP][2][2];
@@ -886,7 +884,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   };
   // basemul-accumulate into the accumulator tile, one job per warp at a
   // time, all k^2 loads of A issued first
-  auto basemul_phase = [&](auto kc, int b, int tl, const uint8_t* slotp) {
+  auto basemul_phase = [&](auto kc, int b, int tl, uint8_t* slotp) {
     constexpr int K = decltype(kc)::value;
     constexpr int kJobs = tile_jobs(K);
     const int njobs = P.njobs[b];
@@ -894,27 +892,37 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       const int job = tl * kJobs + jl;
       if (job >= njobs) break;  // warp-uniform
       const int16_t* Aj = P.A[b] + (size_t)job * K * K * 256 + 8 * lane;
-      uint4 a[K][K];
+      constexpr int kRows = K == 4 ? 2 : K;  // rows of A in flight
+      uint4 a[kRows][K];
       BasemulOperand bv[K];
+      auto load_a = [&](int i0) {
 #pragma unroll
-      for (int i = 0; i < K; i++)
+        for (int i = 0; i < kRows; i++)
 #pragma unroll
-        for (int j = 0; j < K; j++) a[i][j] = __ldcs((const uint4*)(Aj + (i * K + j) * 256));
+          for (int j = 0; j < K; j++)
+            a[i][j] = __ldcs((const uint4*)(Aj + ((i0 + i) * K + j) * 256));
+      };
+      load_a(0);
 #pragma unroll
       for (int j = 0; j < K; j++)
         bv[j] = basemul_operand(*(const uint4*)(slotp + (jl * K + j) * kRowBytes + 16 * lane), zt);
+      __syncwarp();  // every lane has read the job's rows
 #pragma unroll
-      for (int i = 0; i < K; i++) {
-        uint2 even, odd;
-        basemul_row_z<K>(a[i], bv, &even, &odd);
-        uint8_t* const row = accp + (jl * K + i) * kRowBytes;
-        *(uint2*)(row + acc_even) = even;
-        *(uint2*)(row + acc_odd) = odd;
+      for (int i0 = 0; i0 < K; i0 += kRows) {
+        if (i0 > 0) load_a(i0);
+#pragma unroll
+        for (int i = 0; i < kRows; i++) {
+          uint2 even, odd;
+          basemul_row_z<K>(a[i], bv, &even, &odd);
+          uint8_t* const row = slotp + (jl * K + i0 + i) * kRowBytes;
+          *(uint2*)(row + acc_even) = even;
+          *(uint2*)(row + acc_odd) = odd;
+        }
       }
     }
   };
   // inverse NTT plus e on the accumulator tile, in place; then the store
-  auto inv_phase = [&](auto nc, int b, int row0, int nvec) {
+  auto inv_phase = [&](auto nc, uint32_t acc, uint8_t* accp, int b, int row0, int nvec) {
     constexpr int NU = decltype(nc)::value;
     {
       uint32_t iac[PP][2][2][2];
@@ -949,8 +957,6 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       break;
     }
     prefetch(k);
-    // the other slot held tile k-1's s, finished before the barrier above
-    if (k + 1 < nmine) issue_load(k + 1, slot_i ^ 1);
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), tl = t - P.first_tile[b];
     const int kb = P.k[b];  // CTA-uniform
     const int row0 = tl * 8 * tile_units(kb), nvec = P.njobs[b] * kb;
@@ -958,7 +964,11 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       fwd_phase(U3{}, slot, slotp);
     else
       fwd_phase(U4{}, slot, slotp);
-    if (lane == 0) bulk_wait_read<0>();  // the accumulators' last store has been read out
+    if (k + 1 < nmine) {
+      // the other slot held tile k-1: its store (this lane's own box) has been read out
+      if (lane == 0) bulk_wait_read<0>();
+      issue_load(k + 1, slot_i ^ 1);
+    }
     cta_sync_named();
     switch (kb) {
       case 2: basemul_phase(std::integral_constant<int, 2>{}, b, tl, slotp); break;
@@ -967,9 +977,9 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     }
     cta_sync_named();
     if (tile_units(kb) == 3)  // the phase code for the tile's unit count
-      inv_phase(U3{}, b, row0, nvec);
+      inv_phase(U3{}, slot, slotp, b, row0, nvec);
     else
-      inv_phase(U4{}, b, row0, nvec);
+      inv_phase(U4{}, slot, slotp, b, row0, nvec);
   }
   if (lane == 0) bulk_wait_all();
 }
