@@ -274,7 +274,7 @@ __device__ __forceinline__ void poly_stage_inv_wide(uint32_t irow0, uint8_t* min
 // Inverse with kAdd only: polynomial p of this warp (global index poly0 + p)
 // gets addend[poly0 + p] added to its output; the addend words for
 // polynomial p+1 are fetched while p is computed.
-template <bool kInverse, bool kAdd = false>
+template <bool kInverse, bool kAdd = false, int kRows = 8>
 __device__ __forceinline__ void poly_stage(uint32_t mine, uint8_t* minep, uint32_t ldt_off,
                                            const uint32_t (&am)[2][4], int32_t cm_lo,
                                            int32_t cm_hi, const int32_t (&cb)[2][4],
@@ -297,9 +297,9 @@ __device__ __forceinline__ void poly_stage(uint32_t mine, uint8_t* minep, uint32
   ldsm_x4_t(mine + ldt_off, b[0], b[1], b[2], b[3]);
   load_add(0, e);
 #pragma unroll
-  for (int p = 0; p < 8; p++) {
+  for (int p = 0; p < kRows; p++) {
     uint32_t n[4] = {0, 0, 0, 0}, en[4] = {0, 0, 0, 0};
-    if (p < 7) {
+    if (p + 1 < kRows) {
       ldsm_x4_t(mine + (p + 1) * kRowBytes + ldt_off, n[0], n[1], n[2], n[3]);
       load_add(p + 1, en);
     }
@@ -708,16 +708,17 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
 // consecutive jobs of one batch, i.e. kRows(k) = kJobs * k consecutive vector
 // rows of its s / e / out (32 for k = 2, 4; 24 for k = 3): 8-row TMA boxes in,
 // the forward NTT in place (the batch kernels' stages: by polynomial, CTA
-// barrier, by block over the tile's n-tiles), the basemul-accumulate by job
-// (warp w: jobs w, w+4, ...; ntt(s) from shared memory, all k^2 loads of A from
-// global memory issued first, A and e prefetched into L2 one tile ahead with
-// bulk prefetches), the inverse NTT plus e in place on the accumulator tile (e
-// read in stage B, as the batch inverse with addend), 8-row TMA boxes out.
+// barrier, by block over the tile's n-tiles), the basemul-accumulate by job in
+// place over ntt(s) (warp w: jobs w, w+4, ...; a job's rows are read whole before
+// the first is written; its loads of A are issued first, for k = 4 half of them
+// at a time; A and e are prefetched into L2 as the tile starts), the inverse NTT
+// plus e in place (e read in stage B, as the batch inverse with addend), 8-row
+// TMA boxes out.
 // Tiles are numbered across the batches (batch b owns [first_tile[b],
 // first_tile[b+1])) and CTA c takes tiles c, c + G, c + 2G, ... (G CTAs), so
-// the launch has one tail for all batches and its CTAs run one k at a time.  s tiles are double-buffered (the next
-// tile's load runs under this tile's work); the accumulator tile is reused
-// once its previous store has been read out.  Rows past a batch are out of
+// the launch has one tail for all batches and its CTAs run one k at a time.
+// Two slots: the next tile's s loads into the other one once the store of the
+// tile before has been read out of it.  Rows past a batch are out of
 // bounds of its tensor maps (zero-filled in; boxes that start past it are
 // neither loaded nor stored) and jobs past it are skipped.  The stage
 // constants are re-read from L1 at each stage, so that between stages their
@@ -728,7 +729,11 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
 // intermediate's form is this kernel's own: ntt(s) reduced lazily, A words
 // multiplied packed (dp2a), the accumulators written parity-split and unbiased
 // for stage A, e added as packed pairs.  65,536 jobs, k ~ U{2,3,4}: 143.8 ->
-// 133.3 us (4.7 TB/s of A, s, e and out); 1,023 jobs 7.8 -> 7.05 us.
+// 133.3 us; 1,023 jobs 7.8 -> 7.05 us.  The basemul in place (two slots of 17 KB
+// instead of three, the rest left to L1) and k = 4's A in two halves: 133.3 ->
+// 129.4 us; in a seconds-long loop, where the 1 kW limit holds the clock and
+// energy counts, 140.1 -> 136.2.  Five or six CTAs per SM at 96 or 80 registers:
+// 133.2 / 132.6 us.
 struct MvTiles {
   CUtensorMap s_map[kMaxSegs];    // s rows [njobs * k][128 words], 8 x 132-word boxes
   CUtensorMap out_map[kMaxSegs];  // out rows, the same shape (may equal s_map: in place)
@@ -882,8 +887,8 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     load_ac(g_fwd.s2, fac);
     block_stage<true, true, W, PP, NU>(slot, slotp, blk0, ldc_split, stc_off, fac, zc);
   };
-  // basemul-accumulate into the accumulator tile, one job per warp at a
-  // time, all k^2 loads of A issued first
+  // basemul-accumulate in place, one job per warp at a time, its loads of A
+  // issued first (k = 4: half of them, which leaves registers and loses no time)
   auto basemul_phase = [&](auto kc, int b, int tl, uint8_t* slotp) {
     constexpr int K = decltype(kc)::value;
     constexpr int kJobs = tile_jobs(K);
@@ -921,7 +926,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       }
     }
   };
-  // inverse NTT plus e on the accumulator tile, in place; then the store
+  // inverse NTT plus e on the accumulators, in place; then the store
   auto inv_phase = [&](auto nc, uint32_t acc, uint8_t* accp, int b, int row0, int nvec) {
     constexpr int NU = decltype(nc)::value;
     {
