@@ -732,7 +732,9 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
 // 133.3 us; 1,023 jobs 7.8 -> 7.05 us.  The basemul in place (two slots of 17 KB
 // instead of three, the rest left to L1) and k = 4's A in two halves: 133.3 ->
 // 129.4 us; in a seconds-long loop, where the 1 kW limit holds the clock and
-// energy counts, 140.1 -> 136.2.  Five or six CTAs per SM at 96 or 80 registers:
+// energy counts, 140.1 -> 136.2.  A 24-row tile's polynomial stages on all four
+// warps, six rows each, instead of eight on three: k = 3 alone 70.2 -> 66.4 us,
+// the mix 129.6 -> 126.3.  Five or six CTAs per SM at 96 or 80 registers:
 // 133.2 / 132.6 us.
 struct MvTiles {
   CUtensorMap s_map[kMaxSegs];    // s rows [njobs * k][128 words], 8 x 132-word boxes
@@ -874,13 +876,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   // forward NTT of the s tile (in the given slot), in place
   auto fwd_phase = [&](auto nc, uint32_t slot, uint8_t* slotp) {
     constexpr int NU = decltype(nc)::value;
-    if (warp < NU) {
+    {
       uint32_t fam[2][4];
       load_am(g_fwd.s1, fam);
       const uint2 c1 = ldg_keep_u2(&g_fwd.c1[lane][0]);
       const int32_t cbz[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-      poly_stage<false>(slot + 8 * warp * kRowBytes, slotp + 8 * warp * kRowBytes, ldt_off, fam,
-                        (int32_t)c1.x, (int32_t)c1.y, cbz, w_even, w_odd, 0, nullptr, 0, 0, 0);
+      constexpr int kR = 2 * NU;  // rows per warp
+      poly_stage<false, false, kR>(slot + kR * warp * kRowBytes, slotp + kR * warp * kRowBytes,
+                                   ldt_off, fam, (int32_t)c1.x, (int32_t)c1.y, cbz, w_even, w_odd,
+                                   0, nullptr, 0, 0, 0);
     }
     cta_sync_named();
     uint32_t fac[PP][2][2][2];
@@ -935,17 +939,20 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       block_stage<true, true, W, PP, NU>(acc, accp, blk0, ldc_split, stc_inv, iac, zc);
     }
     cta_sync_named();
-    if (warp < NU) {
-      uint32_t iam[2][4];
-      load_am(g_tile_inv.sb, iam);
-      const int32_t cbz[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-      poly_stage<true, true>(acc + 8 * warp * kRowBytes, accp + 8 * warp * kRowBytes, ldt_inv, iam,
-                             0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + 8 * warp, nvec, 8u * g8 + q4);
-      fence_proxy_async_smem();
+    constexpr int kR = 2 * NU;  // rows per warp
+    uint32_t iam[2][4];
+    load_am(g_tile_inv.sb, iam);
+    const int32_t cbz[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    poly_stage<true, true, kR>(acc + kR * warp * kRowBytes, accp + kR * warp * kRowBytes, ldt_inv,
+                               iam, 0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + kR * warp, nvec,
+                               8u * g8 + q4);
+    fence_proxy_async_smem();
+    if (NU == W)
       __syncwarp();
-      if (lane == 0 && row0 + 8 * warp < nvec)  // boxes past the batch are dropped
-        tma_store_2d(&P.out_map[b], 0, row0 + 8 * warp, acc + warp * kWarpBoxBytes);
-    }
+    else
+      cta_sync_named();  // a box's rows come from two warps
+    if (lane == 0 && warp < NU && row0 + 8 * warp < nvec)  // boxes past the batch are dropped
+      tma_store_2d(&P.out_map[b], 0, row0 + 8 * warp, acc + warp * kWarpBoxBytes);
     if (lane == 0) bulk_commit();  // every lane-0 keeps one (possibly empty) group per tile
   };
   using U3 = std::integral_constant<int, 3>;
