@@ -170,20 +170,20 @@ __device__ __forceinline__ void block_stage(uint32_t slot, uint8_t* slotp, int b
 // block_stage, two ldmatrix.x4 per block pair (one per block).  ldw[p]: this
 // lane's ldmatrix row offset of pair p's first block (polynomial lane&7 of
 // the n-tile, parity (lane/16) placed by the row swizzle, half (lane/8)&1).
-template <int W, int P>
+template <int NT, int P>
 __device__ __forceinline__ void block_stage_wide(uint32_t inter, uint8_t* slotp, int blk0,
                                                  const uint32_t (&ldw)[P], uint32_t stc_off,
                                                  const uint32_t (&ac)[P][2][2][4]) {
-  constexpr int kIters = P * W;
+  constexpr int kIters = P * NT;
   uint32_t r[8];
   ldsm_x4(inter + ldw[0], r[0], r[1], r[2], r[3]);
   ldsm_x4(inter + ldw[0] + 64, r[4], r[5], r[6], r[7]);
 #pragma unroll
   for (int it = 0; it < kIters; it++) {
-    const int p = it / W, nt = it % W;
+    const int p = it / NT, nt = it % NT;
     uint32_t n[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (it + 1 < kIters) {
-      const int p1 = (it + 1) / W, nt1 = (it + 1) % W;
+      const int p1 = (it + 1) / NT, nt1 = (it + 1) % NT;
       const uint32_t a1 = inter + nt1 * 8 * kWideRowBytes + ldw[p1];
       ldsm_x4(a1, n[0], n[1], n[2], n[3]);
       ldsm_x4(a1 + 64, n[4], n[5], n[6], n[7]);
@@ -197,21 +197,21 @@ __device__ __forceinline__ void block_stage_wide(uint32_t inter, uint8_t* slotp,
 // Inverse stage A of one tile into the int32 intermediates (wide kernels): as
 // block_stage<true>, the sums of pair p stored at offsets ia[p][s] of the rows
 // of polynomials 2q, 2q+1 of each n-tile.
-template <int W, int P>
+template <int NT, int P>
 __device__ __forceinline__ void block_stage_inv_wide(uint32_t slot, int blk0, uint32_t ldc_off,
                                                      uint8_t* interp, uint32_t row_off,
                                                      const uint32_t (&ia)[P][2],
                                                      const uint32_t (&ac)[P][2][2][2],
                                                      const int32_t (&cc)[P][2][2]) {
-  constexpr int kIters = P * W;
+  constexpr int kIters = P * NT;
   uint32_t r[4];
   ldsm_x4(slot + 32u * blk0 + ldc_off, r[0], r[1], r[2], r[3]);
 #pragma unroll
   for (int it = 0; it < kIters; it++) {
-    const int p = it / W, nt = it % W;
+    const int p = it / NT, nt = it % NT;
     uint32_t n[4] = {0, 0, 0, 0};
     if (it + 1 < kIters) {
-      const int p1 = (it + 1) / W, nt1 = (it + 1) % W;
+      const int p1 = (it + 1) / NT, nt1 = (it + 1) % NT;
       ldsm_x4(slot + nt1 * 8 * kRowBytes + 32u * (blk0 + 2 * p1) + ldc_off, n[0], n[1], n[2],
               n[3]);
     }
@@ -228,7 +228,7 @@ __device__ __forceinline__ void block_stage_inv_wide(uint32_t slot, int blk0, ui
 // Inverse stage B of this warp's 8 polynomials from the int32 intermediates
 // (wide kernels; irow0: the first one's row), two ldmatrix.x4 per polynomial,
 // the next one's issued ahead; addend as poly_stage.
-template <bool kAdd>
+template <bool kAdd, int kRows = 8>
 __device__ __forceinline__ void poly_stage_inv_wide(uint32_t irow0, uint8_t* minep,
                                                     const uint32_t (&lb)[2],
                                                     const uint32_t (&a)[2][2][4],
@@ -252,9 +252,9 @@ __device__ __forceinline__ void poly_stage_inv_wide(uint32_t irow0, uint8_t* min
   ldsm_x4(irow0 + lb[1], b[1][0], b[1][1], b[1][2], b[1][3]);
   load_add(0, e);
 #pragma unroll
-  for (int p = 0; p < 8; p++) {
+  for (int p = 0; p < kRows; p++) {
     uint32_t n[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, en[4] = {0, 0, 0, 0};
-    if (p < 7) {
+    if (p + 1 < kRows) {
       const uint32_t nx = irow0 + (p + 1) * kWideRowBytes;
       ldsm_x4(nx + lb[0], n[0][0], n[0][1], n[0][2], n[0][3]);
       ldsm_x4(nx + lb[1], n[1][0], n[1][1], n[1][2], n[1][3]);
@@ -325,7 +325,7 @@ __device__ __forceinline__ void poly_stage(uint32_t mine, uint8_t* minep, uint32
 // m = 2t, 2t+1, 8+2t, 9+2t.  Output to minep's rows (kRowBytes apart,
 // parity-split int16), or with kWideOut unreduced to int32 intermediate rows
 // (kWideRowBytes apart; w_even / w_odd then the wide offsets).
-template <int kIn, bool kWideOut = false>
+template <int kIn, bool kWideOut = false, int kRows = 8>
 __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, uint32_t ldt_off,
                                                  const uint8_t* packp, const uint32_t (&ab)[2][2],
                                                  int32_t cb_lo, int32_t cb_hi, uint32_t w_even,
@@ -342,9 +342,9 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
     uint32_t b[4];
     ldsm_x4_t(mine + ldt_off, b[0], b[1], b[2], b[3]);
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
+    for (int p = 0; p < kRows; p++) {
       uint32_t nx[4] = {0, 0, 0, 0};
-      if (p < 7) ldsm_x4_t(mine + (p + 1) * kRowBytes + ldt_off, nx[0], nx[1], nx[2], nx[3]);
+      if (p + 1 < kRows) ldsm_x4_t(mine + (p + 1) * kRowBytes + ldt_off, nx[0], nx[1], nx[2], nx[3]);
       const uint32_t bt0 = small_operand(b[0], b[1], bad);
       const uint32_t bt1 = small_operand(b[2], b[3], bad);
       out(p, bt0, bt1);
@@ -358,7 +358,7 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
     const uint32_t sel0 = k0 | ((k0 + 4) << 4), sel1 = k1 | ((k1 + 4) << 4);
     const uint32_t shift = 2 * (n & 3);
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
+    for (int p = 0; p < kRows; p++) {
       const uint8_t* pk = packp + p * 64;
       const uint2 v01 = *(const uint2*)(pk + 8 * t);       // m = 2t, 2t+1
       const uint2 v23 = *(const uint2*)(pk + 32 + 8 * t);  // m = 8+2t, 9+2t
@@ -373,7 +373,7 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
     const uint32_t sel = k | ((k + 4) << 4);
     const uint32_t shift = 3 * (n & 1);
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
+    for (int p = 0; p < kRows; p++) {
       const uint8_t* pk = packp + p * 128;
       const uint4 v01 = *(const uint4*)(pk + 16 * t);       // m = 2t, 2t+1
       const uint4 v23 = *(const uint4*)(pk + 64 + 16 * t);  // m = 8+2t, 9+2t
@@ -381,6 +381,25 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
       const uint32_t bt1 = packed_operand<3>(v01.y, v01.w, v23.y, v23.w, sel, shift);
       out(p, bt0, bt1);
     }
+  }
+}
+
+// Forward stage 1 of kRows polynomials into the int32 intermediates (wide
+// kernels), the next ldmatrix issued ahead.
+template <int kRows = 8>
+__device__ __forceinline__ void poly_stage_fwd_wide(uint32_t rows, uint8_t* irows, uint32_t ldt_off,
+                                                    const uint32_t (&am)[2][4], int32_t cm_lo,
+                                                    int32_t cm_hi, uint32_t wi_e, uint32_t wi_o) {
+  uint32_t b[4];
+  ldsm_x4_t(rows + ldt_off, b[0], b[1], b[2], b[3]);
+#pragma unroll
+  for (int p = 0; p < kRows; p++) {
+    uint32_t n[4] = {0, 0, 0, 0};
+    if (p + 1 < kRows) ldsm_x4_t(rows + (p + 1) * kRowBytes + ldt_off, n[0], n[1], n[2], n[3]);
+    stage_m_wide(am, cm_lo, cm_hi, b[0] ^ 0x80008000u, b[1] ^ 0x80008000u, b[2] ^ 0x80008000u,
+                 b[3] ^ 0x80008000u, irows + p * kWideRowBytes, wi_e, wi_o);
+#pragma unroll
+    for (int j = 0; j < 4; j++) b[j] = n[j];
   }
 }
 
@@ -595,6 +614,57 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
     bulk_commit();
   };
 
+  // A tile of at most 3/4 W units, the last one of a CTA's run, computed as a
+  // quarter, half or three quarters of a tile (four warps: exactly its units):
+  // the stages over m spread its polynomials over all W warps, the block-wise
+  // stages run fewer n-tiles.  Computing such a tile whole cost a full
+  // tile's time (about 2 us at four CTAs per SM) for as little as one unit:
+  // forward, us, 1,000 polynomials 2.58 -> 1.77, 16,411 6.33 -> 4.91, 100,003
+  // 22.1 -> 21.2, 262,144 49.6 -> 48.7; inverse (variant 0) 40,009 13.9 -> 11.8,
+  // 100,003 25.0 -> 23.1.  Unrolled for each size: as loops over units 6,000
+  // polynomials took 3.13 instead of 3.01 us (262,144: 48.4).
+  constexpr bool kShortTile = !kMulti && !kAdd;
+  auto short_tile = [&](auto nc, uint32_t slot, uint8_t* slotp) {
+    constexpr int NU = decltype(nc)::value, R = NU * 8 / W;
+    const int row = R * warp;  // this warp's first row in the stages over m
+    const uint32_t rows = slot + row * kRowBytes;
+    uint8_t* const rowsp = slotp + row * kRowBytes;
+    if constexpr (kInverse) {
+      if constexpr (kWide)
+        block_stage_inv_wide<NU>(slot, blk0, ldc_off, interp, ia_row, ia, ac, cc);
+      else
+        block_stage<false, true, W, C::kPairsPerWarp, NU>(slot, slotp, blk0, ldc_off, stc_off, ac,
+                                                          cc);
+      cta_sync_named();
+      if constexpr (kWide)
+        poly_stage_inv_wide<false, R>(inter + row * kWideRowBytes, rowsp, lb, amw, cb, w_nat,
+                                      nullptr, 0, 0, 0);
+      else
+        poly_stage<true, false, R>(rows, rowsp, ldt_off, am, cm_lo, cm_hi, cb, 0, 0, w_nat, nullptr,
+                                   0, 0, 0);
+    } else {
+      uint8_t* const dst = kWide ? interp + row * kWideRowBytes : rowsp;
+      if constexpr (kIn != kInInt16)
+        poly_stage_small<kIn, kWide, R>(rows, dst, ldt_off,
+                                        slotp + C::kRowsBytes + row * C::kPackBytes, ab, cb_lo,
+                                        cb_hi, kWide ? wi_e : w_even, kWide ? wi_o : w_odd, lane,
+                                        &bad);
+      else if constexpr (kWide)
+        poly_stage_fwd_wide<R>(rows, dst, ldt_off, am, cm_lo, cm_hi, wi_e, wi_o);
+      else
+        poly_stage<false, false, R>(rows, rowsp, ldt_off, am, cm_lo, cm_hi, cb, w_even, w_odd, 0,
+                                    nullptr, 0, 0, 0);
+      cta_sync_named();
+      if constexpr (kWide)
+        block_stage_wide<NU>(inter, slotp, blk0, ldw, stc_off, ac);
+      else
+        block_stage<true, false, W, C::kPairsPerWarp, NU>(slot, slotp, blk0, ldc_off, stc_off, ac,
+                                                          cc);
+    }
+    fence_proxy_async_smem();
+    cta_sync_named();  // a box's rows come from every warp
+  };
+
   // prologue: tiles 0 .. S-2 into slots 0 .. S-2
 #pragma unroll
   for (int t = 0; t < C::kSlots - 1; t++)
@@ -623,6 +693,19 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
     const uint32_t mine = slot + 8 * warp * kRowBytes;
     uint8_t* minep = slotp + 8 * warp * kRowBytes;
 
+    if constexpr (kShortTile) {
+      const int nu = u_end - (u_begin + k * W);  // live units; CTA-uniform
+      if (nu <= 3 * W / 4) {  // the CTA's last tile
+        if (nu <= W / 4)
+          short_tile(std::integral_constant<int, W / 4>{}, slot, slotp);
+        else if (nu <= W / 2)
+          short_tile(std::integral_constant<int, W / 2>{}, slot, slotp);
+        else
+          short_tile(std::integral_constant<int, 3 * W / 4>{}, slot, slotp);
+        issue_store(k, slot_i);
+        break;
+      }
+    }
     if constexpr (kWide && kInverse) {
       block_stage_inv_wide<W>(slot, blk0, ldc_off, interp, ia_row, ia, ac, cc);
       cta_sync_named();
@@ -636,18 +719,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
     } else if constexpr (kWide) {
       uint8_t* irow0 = interp + 8 * warp * kWideRowBytes;
       if constexpr (kIn == kInInt16) {
-        uint32_t b[4];
-        ldsm_x4_t(mine + ldt_off, b[0], b[1], b[2], b[3]);
-#pragma unroll
-        for (int p = 0; p < 8; p++) {
-          uint32_t n[4] = {0, 0, 0, 0};
-          if (p < 7) ldsm_x4_t(mine + (p + 1) * kRowBytes + ldt_off, n[0], n[1], n[2], n[3]);
-          stage_m_wide(am, cm_lo, cm_hi, b[0] ^ 0x80008000u, b[1] ^ 0x80008000u,
-                       b[2] ^ 0x80008000u, b[3] ^ 0x80008000u, irow0 + p * kWideRowBytes, wi_e,
-                       wi_o);
-#pragma unroll
-          for (int j = 0; j < 4; j++) b[j] = n[j];
-        }
+        poly_stage_fwd_wide(mine, irow0, ldt_off, am, cm_lo, cm_hi, wi_e, wi_o);
       } else {
         uint32_t tile_bad = 0;  // as below: only live rows count
         poly_stage_small<kIn, true>(mine, irow0, ldt_off,
@@ -1001,7 +1073,11 @@ struct Variant {
   const void* fn;
   int threads;
   int smem;
-  int tile;
+  int tile;   // polynomials per tile
+  // CTAs are launched for at least this many polynomials: one unit where short
+  // tiles cost less than whole ones (1,000 polynomials on 125 CTAs 1.77 us, on 32
+  // CTAs 2.53), else a tile
+  int grain;
 };
 
 template <bool I, int W, int S, int kIn = kInInt16, bool kAdd = false, class P = OneSeg,
@@ -1009,7 +1085,7 @@ template <bool I, int W, int S, int kIn = kInInt16, bool kAdd = false, class P =
 constexpr Variant make_variant() {
   using C = Cfg<W, S, kIn, kWide>;
   return Variant{(const void*)k_ntt_mma<I, W, S, kIn, kAdd, P, kWide>, C::kThreads, C::kSmem,
-                 C::kTile};
+                 C::kTile, kAdd || std::is_same<P, SegMaps>::value ? C::kTile : 8};
 }
 
 // [inverse][variant] (the mma.sync variants; variant 4 is tk_tc5.cu's)
@@ -1190,7 +1266,7 @@ bool mma_init_device(DeviceInfo* info) {
 template <class P>
 static cudaError_t launch_variant(const Variant& V, long long cap, const P& m, long long polys,
                                   cudaStream_t stream) {
-  long long ctas = (polys + V.tile - 1) / V.tile;
+  long long ctas = (polys + V.grain - 1) / V.grain;
   if (ctas > cap) ctas = cap;
   if (ctas < 1) ctas = 1;
   cudaLaunchConfig_t cfg = {};
