@@ -440,11 +440,13 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
   // block-wise stage accumulator init: zero (the inverse's stage-A bias
   // offset is cancelled by stage B's init cb instead)
   int32_t cc[C::kPairsPerWarp][2][2];
-  int32_t cb[2][4];  // inverse stage B: group-0 init per n-tile (InvFrags::cbz)
+  // inverse stage B: group-0 init per n-tile (InvFrags::cbz), plus what the
+  // centred reduction expects on its sums
+  int32_t cb[2][4];
 #pragma unroll
   for (int t = 0; t < 2; t++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) cb[t][j] = kInverse ? g_inv.cbz[lane][t][j] : 0;
+    for (int j = 0; j < 4; j++) cb[t][j] = kInverse ? g_inv.cbz[lane][t][j] + kCentre : 0;
   const int blk0 = C::kBlocksPerWarp * warp;
 #pragma unroll
   for (int g = 0; g < 2; g++)
@@ -1014,7 +1016,8 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     constexpr int kR = 2 * NU;  // rows per warp
     uint32_t iam[2][4];
     load_am(g_tile_inv.sb, iam);
-    const int32_t cbz[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    const int32_t cbz[2][4] = {{kCentre, kCentre, kCentre, kCentre},
+                               {kCentre, kCentre, kCentre, kCentre}};
     poly_stage<true, true, kR>(acc + kR * warp * kRowBytes, accp + kR * warp * kRowBytes, ldt_inv,
                                iam, 0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + kR * warp, nvec,
                                8u * g8 + q4);

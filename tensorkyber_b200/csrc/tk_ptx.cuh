@@ -177,26 +177,39 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ uint32_t red_lazy(uint32_t s) {
   return s - __umulhi(s, 1290167u) * 3329u;
 }
-// S in [0, 2^26): canonical representative in [0, q).
-__device__ __forceinline__ uint32_t red_exact(uint32_t s) {
-  return s - (__umulhi(s, 82570715u) >> 6) * 3329u;
-}
 // S + (q-1)/2 < 2^26: the centred representative of S mod q, in
 // [-(q-1)/2, (q-1)/2] (two's complement): floor((S + 1664) / q) by
-// red_exact's multiplier, the offset folded into the 64-bit product's addend
+// multiplication by ceil(2^38 / q), the offset folded into the 64-bit product's addend
 // (one multiply-add), so no separate add or subtract of 1664.
 __device__ __forceinline__ uint32_t red_centred(uint32_t s) {
   const uint64_t x = (uint64_t)s * 82570715ull + 1664ull * 82570715ull;
   return s - (uint32_t)(x >> 38) * 3329u;
-}
-__device__ __forceinline__ uint32_t pack2(uint32_t lo, uint32_t hi) {
-  return __byte_perm(lo, hi, 0x5410);
 }
 // Two int16 additions, each wrapping.
 __device__ __forceinline__ uint32_t add16x2(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("add.s16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
+}
+// Two sums below 2^26 -> the packed pair of their canonical residues.  The
+// quotients floor(S / q) = (S * ceil(2^40 / q)) >> 40 (exact: S e < 2^40, e =
+// 3177) fill bytes 1 and 2 of the products' high words, so one byte permute packs
+// them and one multiply-subtract of the packed quotients finishes both: 5
+// instructions a pair, against 7 for two shifted quotients, two subtractions and
+// a pack2.
+__device__ __forceinline__ uint32_t red_exact_pair(uint32_t s0, uint32_t s1) {
+  constexpr uint32_t kM = 330282857u;
+  const uint32_t q = __byte_perm(__umulhi(s0, kM), __umulhi(s1, kM), 0x6521);
+  return (s0 + (s1 << 16)) - q * 3329u;
+}
+// The sums plus (q-1)/2, below 2^26 (the caller's accumulators start at kCentre)
+// -> the packed pair of the sums' centred representatives.
+constexpr int32_t kCentre = 1664;
+__device__ __forceinline__ uint32_t red_centred_pair(uint32_t s0, uint32_t s1) {
+  return add16x2(red_exact_pair(s0, s1), 0xF980F980u);  // - 1664 each
+}
+__device__ __forceinline__ uint32_t pack2(uint32_t lo, uint32_t hi) {
+  return __byte_perm(lo, hi, 0x5410);
 }
 // c + a.h0 b.b0 + a.h1 b.b1 (lo) or c + a.h0 b.b2 + a.h1 b.b3 (hi): signed
 // halves of a, unsigned bytes of b.

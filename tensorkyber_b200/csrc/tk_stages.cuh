@@ -24,7 +24,8 @@ __device__ __forceinline__ void stage_m_out(const int32_t (&lo0)[4], const int32
 // operands (ldmatrix.trans of the natural-order row) are b0..b3.  Inverse
 // with kAdd: the addend pairs `add` are added to the output (int16
 // wrap-around); without it `add` is ignored.
-// c0 / c1: the group-0 accumulator init of n-tiles 0 and 1 (D register order).
+// c0 / c1: the group-0 accumulator init of n-tiles 0 and 1 (D register order);
+// the inverse's includes kCentre (red_centred_pair).
 template <bool kInverse, bool kAdd = false>
 __device__ __forceinline__ void stage_m_q(const uint32_t (&a)[2][4], const int32_t (&c0)[4],
                                           const int32_t (&c1)[4], uint32_t b0, uint32_t b1,
@@ -50,8 +51,8 @@ __device__ __forceinline__ void stage_m(const uint32_t (&a)[2][4], int32_t c_lo,
 }
 
 // Epilogue of the stage over m from its accumulators (lo / hi limb, n-tiles 0
-// and 1): forward lazy reduction to parity-split rows; inverse exact reduction,
-// centring and (kAdd) the addend, natural order.
+// and 1): forward lazy reduction to parity-split rows; inverse (sums plus kCentre)
+// exact reduction, centring and (kAdd) the addend, natural order.
 template <bool kInverse, bool kAdd>
 __device__ __forceinline__ void stage_m_out(const int32_t (&lo0)[4], const int32_t (&hi0)[4],
                                             const int32_t (&lo1)[4], const int32_t (&hi1)[4],
@@ -60,20 +61,13 @@ __device__ __forceinline__ void stage_m_out(const int32_t (&lo0)[4], const int32
   uint32_t y0[4], y1[4];
 #pragma unroll
   for (int e = 0; e < 4; e++) {
-    const uint32_t s0 = (uint32_t)lo0[e] + ((uint32_t)hi0[e] << 7);
-    const uint32_t s1 = (uint32_t)lo1[e] + ((uint32_t)hi1[e] << 7);
-    if (kInverse) {  // centred
-      y0[e] = red_centred(s0);
-      y1[e] = red_centred(s1);
-    } else {
-      y0[e] = red_lazy(s0);
-      y1[e] = red_lazy(s1);
-    }
+    y0[e] = (uint32_t)lo0[e] + ((uint32_t)hi0[e] << 7);
+    y1[e] = (uint32_t)lo1[e] + ((uint32_t)hi1[e] << 7);
   }
   // D regs: [0] (row i, c=2q), [1] (row i, c=2q+1), [2]/[3] row i+8; n-tile 1 is c+8.
   if (kInverse) {  // natural order; plus the addend pairs (int16 wrap-around add)
-    uint32_t w[4] = {pack2(y0[0], y0[1]), pack2(y1[0], y1[1]), pack2(y0[2], y0[3]),
-                     pack2(y1[2], y1[3])};
+    uint32_t w[4] = {red_centred_pair(y0[0], y0[1]), red_centred_pair(y1[0], y1[1]),
+                     red_centred_pair(y0[2], y0[3]), red_centred_pair(y1[2], y1[3])};
     if (kAdd) {
 #pragma unroll
       for (int j = 0; j < 4; j++) w[j] = add16x2(w[j], add[j]);
@@ -83,6 +77,11 @@ __device__ __forceinline__ void stage_m_out(const int32_t (&lo0)[4], const int32
     *(uint32_t*)(row + w_nat + 256) = w[2];
     *(uint32_t*)(row + w_nat + 256 + 16) = w[3];
   } else {  // parity-split slots (c=2q | c=8+2q), (c=2q+1 | c=9+2q)
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      y0[e] = red_lazy(y0[e]);
+      y1[e] = red_lazy(y1[e]);
+    }
     *(uint32_t*)(row + w_even) = pack2(y0[0], y1[0]);
     *(uint32_t*)(row + w_odd) = pack2(y0[1], y1[1]);
     *(uint32_t*)(row + w_even + 256) = pack2(y0[2], y1[2]);
@@ -241,14 +240,13 @@ __device__ __forceinline__ void stage_c(const uint32_t (&a)[2][2][2], const int3
     const uint32_t se1 = (uint32_t)de[1] + ((uint32_t)de[3] << 7);
     const uint32_t so0 = (uint32_t)dodd[0] + ((uint32_t)dodd[2] << 7);
     const uint32_t so1 = (uint32_t)dodd[1] + ((uint32_t)dodd[3] << 7);
-    uint32_t e0, e1, o0, o1;
     if (kLazy) {
-      e0 = red_lazy(se0); e1 = red_lazy(se1); o0 = red_lazy(so0); o1 = red_lazy(so1);
+      *(uint32_t*)(out + 32 * h) = pack2(red_lazy(se0), red_lazy(so0));
+      *(uint32_t*)(out + kRowBytes + 32 * h) = pack2(red_lazy(se1), red_lazy(so1));
     } else {
-      e0 = red_exact(se0); e1 = red_exact(se1); o0 = red_exact(so0); o1 = red_exact(so1);
+      *(uint32_t*)(out + 32 * h) = red_exact_pair(se0, so0);
+      *(uint32_t*)(out + kRowBytes + 32 * h) = red_exact_pair(se1, so1);
     }
-    *(uint32_t*)(out + 32 * h) = pack2(e0, o0);
-    *(uint32_t*)(out + kRowBytes + 32 * h) = pack2(e1, o1);
   }
 }
 
@@ -265,12 +263,11 @@ __device__ __forceinline__ void stage_c_wide(const uint32_t (&a)[2][2][4], const
     int32_t de[4], dodd[4];
     mma_k32(de, a[h][0], r[4 * h], r[4 * h + 1], zero);
     mma_k32(dodd, a[h][1], r[4 * h + 2], r[4 * h + 3], zero);
-    const uint32_t e0 = red_exact((uint32_t)de[0] + ((uint32_t)de[2] << 7));
-    const uint32_t e1 = red_exact((uint32_t)de[1] + ((uint32_t)de[3] << 7));
-    const uint32_t o0 = red_exact((uint32_t)dodd[0] + ((uint32_t)dodd[2] << 7));
-    const uint32_t o1 = red_exact((uint32_t)dodd[1] + ((uint32_t)dodd[3] << 7));
-    *(uint32_t*)(out + 32 * h) = pack2(e0, o0);
-    *(uint32_t*)(out + kRowBytes + 32 * h) = pack2(e1, o1);
+    *(uint32_t*)(out + 32 * h) = red_exact_pair((uint32_t)de[0] + ((uint32_t)de[2] << 7),
+                                                (uint32_t)dodd[0] + ((uint32_t)dodd[2] << 7));
+    *(uint32_t*)(out + kRowBytes + 32 * h) =
+        red_exact_pair((uint32_t)de[1] + ((uint32_t)de[3] << 7),
+                       (uint32_t)dodd[1] + ((uint32_t)dodd[3] << 7));
   }
 }
 

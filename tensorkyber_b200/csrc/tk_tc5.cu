@@ -503,8 +503,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
             uint32_t w[8];
 #pragma unroll
             for (int t = 0; t < 8; t++)
-              w[t] = pack2(red_exact(ru[2 * t] + (ru[16 + 2 * t] << 7)),
-                           red_exact(ru[2 * t + 1] + (ru[17 + 2 * t] << 7)));
+              w[t] = red_exact_pair(ru[2 * t] + (ru[16 + 2 * t] << 7),
+                                    ru[2 * t + 1] + (ru[17 + 2 * t] << 7));
             const uint32_t i = 4u * g + 2u * jj + u;
             st_shared_v4(sw128_chunk(slot, p, 2u * i), w[0], w[1], w[2], w[3]);
             st_shared_v4(sw128_chunk(slot, p, 2u * i + 1), w[4], w[5], w[6], w[7]);
