@@ -1289,10 +1289,9 @@ static cudaError_t launch_variant(const Variant& V, long long cap, const P& m, l
 // Packed inputs above two full waves of the mma.sync form's 32-polynomial tiles
 // (28,416 polynomials on 148 SMs) run the dense kernel (tk_pack.cu).  Below,
 // its 128-polynomial tiles leave SMs idle and its longer chain per tile shows:
-// 2-bit, us, mma.sync / dense: 4,096 2.9 / 5.4, 12,000 4.3 / 5.7, 20,011 6.4 /
-// 7.0; above: 32,768 9.4 / 7.5, 100,003 21.7 / 16.0, 262,144 50.1 / 30.0, 2^20
-// 187.1 / 104.7 (3-bit 191.4 / 114.3).
-
+// 2-bit, us, mma.sync / dense: 4,096 2.7 / 5.4, 12,000 3.6 / 5.7, 20,011 5.4 /
+// 7.0; above: 32,768 9.0 / 7.5, 100,003 20.9 / 15.9, 262,144 47.8 / 31.5, 2^20 185
+// / 105-113.
 cudaError_t launch_fwd_form(int form, const void* src, int16_t* dst, long long npoly,
                             const DeviceInfo& info, cudaStream_t stream) {
   if (form < 1 || form > kNumInputForms) return cudaErrorInvalidValue;

@@ -3,44 +3,53 @@
 // product on the 5th-generation tensor cores, sm_100a.
 //
 // The transform never mixes even and odd coefficients, and both halves meet
-// the same 128 x 128 matrix F: out[2t + p] = sum_j F[t][j] x[2j + p].  For
-// coefficients of 2 or 3 bits that product needs no second stage, no second
-// constant limb and no int32 intermediates:
+// the same 128 x 128 matrix F: out[2t + p] = sum_j F[t][j] x[2j + p].  Rows 2m and
+// 2m + 1 of F belong to roots z and -z, so F is 64 rows over even j (P) and 64
+// over odd j (M) with outputs P + M and P - M.  For coefficients of 2 or 3 bits
+// that needs no second stage, no second constant limb and no int32
+// intermediates:
 //
-//   * A constant c, centred in [-(q-1)/2, (q-1)/2], is c0 + 2^s c1 (s = 8 -
-//     bits) with both parts int8.  The data side carries the coefficient
-//     twice, as x and as 2^s x -- the packed field moved to the top of a byte
-//     -- so one signed K run holds both and the accumulator is the sum itself:
-//     128 outputs per parity, K = 256 bytes, |S| <= 128 * 4 * 1664 < 2^20.
-//   * The operand goes from the packed words straight to tensor memory: two
-//     table look-ups (__byte_perm) per four 2-bit fields, or a mask and a
-//     multiply-add per four 3-bit ones.  Nothing is staged in shared memory.
+//   * A constant c is, mod q, c0 + 2^s c1 (s = 8 - bits) with both parts int8.
+//     The data side carries the coefficient twice, as x + 2^(bits-1) -- the field
+//     with its sign bit flipped -- and as 2^s x, the field moved to the top of a
+//     byte, so one signed K run holds both and the accumulator is the sum itself:
+//     64 sums per part and parity, K = 128 bytes.  Every row's c0 sum to zero, so
+//     the offset of the first form adds nothing; its small bytes toggle less
+//     of the multipliers than sign-extended ones.  |P +- M| < 2^20.
+//   * The operand goes from the packed words straight to tensor memory, a mask, an
+//     exclusive or and a shift per two operand words.  Nothing is staged in shared
+//     memory.
 //   * One exact reduction per output, in the pair: the quotients are the high
 //     words of S * ceil(2^32 / q) + 2^31 / q (exact floors for either sign in
 //     this range), and S0 + 2^16 S1 - q (q0 + 2^16 q1) is the packed pair, 2.5
 //     instructions per coefficient.
 //
-// What bounds it: the memory, mostly its writes.  2^20 polynomials of 2-bit
-// fields take 104.7 us, 5.8 TB/s (0.88 of a measured copy); the mma.sync form
-// took 187.1 us, issuing 103 warp-instructions per polynomial for two matrix
-// stages with fragments through shared memory, however small its input.
+// What bounds it: the memory, mostly its writes, and in a long loop the 1 kW
+// limit.  2^20 polynomials of 2-bit fields take 105-113 us (0.82-0.88 of a
+// measured copy; 123 in a long loop), of 3-bit ones 114; the mma.sync form took
+// 187 and 191, issuing 103 warp-instructions per polynomial for two matrix stages
+// with fragments through shared memory, however small its input.  Energy decides
+// the long loop: issuing every MMA twice cost 20 us there, hence P and M instead
+// of the full matrix (half the products for one addition per output) and the small
+// operand bytes; 3-bit 134 -> 127 us, 262,144 polynomials 36.5 -> 34.6.
 //
 // Tile: 128 polynomials, the M dimension of every MMA (one per tensor-memory
-// lane).  Roles (640 threads, one CTA per SM by shared memory):
-//   warps 0-15   four groups of four (warp w reaches lanes 32 (w % 4) ..):
-//                unpack quarter g of every row of tile k + 1, then read, reduce
-//                and write quarter g of tile k's outputs (pairs 32 g .. + 31)
-//   warps 16, 17 lane 0 issues the MMAs of output half 0 / 1 (64 outputs of
-//                each parity: one issuing thread cannot keep the pipe fed)
-//   warp 18      lane 0 loads packed tiles (and the constants, once)
-//   warp 19      lane 0 stores the output boxes; the first issuer's warp owns
+// lane).  Roles (768 threads, one CTA per SM by shared memory):
+//   warps 0-15   four groups of four (warp w reaches lanes 32 (w % 4) ..): read,
+//                reduce and write quarter g of a tile's outputs (pairs 32 g .. +
+//                31, from P and M rows 16 g .. + 15), eight rows at a time
+//   warps 16-19  unpack, a row per thread, up to two tiles ahead: as part of the
+//                other warps' loop it held the stores back
+//   warps 20, 21 lane 0 issues the MMAs of the even / odd coefficients (one
+//                issuing thread cannot keep the pipe fed)
+//   warp 22      lane 0 loads packed tiles (and the constants, once)
+//   warp 23      lane 0 stores the output boxes; the first issuer's warp owns
 //                the tensor-memory allocation
-// Tensor memory (512 columns): two operand buffers of 128 columns (even,
-// odd: 64 each) at 128 b, and an accumulator buffer of 128 columns per output
-// half (even, odd: 64 each) at 256 + 128 c.  So tile k + 1 is unpacked and
-// multiplied while tile k is reduced, and the stores of tiles k and k - 1
-// drain from two 64 KiB output slots (TMA's 128-byte swizzle layout, boxes of
-// 64 coefficients).
+// Tensor memory (512 columns): two operand buffers of 128 columns (even, odd:
+// P and M parts of 32 each) at 128 b, and 128 accumulator columns per parity (P,
+// M: 64 each) at 256 + 128 p.  So the next tiles are unpacked and multiplied while
+// a tile is reduced, and stores drain from two or three 64 KiB output slots (TMA's
+// 128-byte swizzle layout, boxes of 64 coefficients).
 // Every mbarrier wait gives up after 2 s (status bit 0); the issuers then
 // drain their MMAs and the copy warps their copies before the CTA ends.
 #include <cuda.h>
@@ -61,22 +70,24 @@ constexpr int kPkTile = 128;                       // polynomials per tile (MMA 
 constexpr int kPkOutBox = kPkTile * 128;           // 64 coefficients x 128 rows
 constexpr int kPkOutSlot = 4 * kPkOutBox;          // 64 KiB
 constexpr int kPkEpiWarps = 16;
-constexpr int kPkMmaWarp = 16, kPkLoadWarp = 18, kPkStoreWarp = 19;
-constexpr int kPkThreads = 640;
+constexpr int kPkUnpackWarp = 16, kPkUnpackWarps = 4;
+constexpr int kPkMmaWarp = 20, kPkLoadWarp = 22, kPkStoreWarp = 23;
+constexpr int kPkThreads = 768;
 constexpr uint32_t kPkTmemCols = 512;
 constexpr uint64_t kPkWaitNs = 2000000000ull;
 
 template <int kBits>
 struct PkLayout {
   static constexpr int kRow = kBits == 2 ? 64 : 128;  // packed bytes per polynomial
-  static constexpr int kInSlots = kBits == 2 ? 4 : 3;
+  static constexpr int kInSlots = kBits == 2 ? 2 : 3;
+  static constexpr int kOutSlots = kBits == 2 ? 3 : 2;  // what fits beside the input
   static constexpr int kInBytes = kPkTile * kRow;
   static constexpr int kOffOut = kPackTableBytes;     // 1024-byte aligned
-  static constexpr int kOffIn = kOffOut + 2 * kPkOutSlot;
+  static constexpr int kOffIn = kOffOut + kOutSlots * kPkOutSlot;
   static constexpr int kOffBars = kOffIn + kInSlots * kInBytes;
-  // in_full, in_empty [kInSlots]; x_ready, op_free [2]; d_full, d_empty [2];
-  // out_ready [2][4]; out_free [2]; consts; drain
-  static constexpr int kBars = 2 * kInSlots + 4 + 4 + 8 + 2 + 2;
+  // in_full, in_empty [kInSlots]; x_ready, op_free [2]; d_full; d_empty;
+  // out_ready [kOutSlots][4]; out_free [kOutSlots]; consts; drain
+  static constexpr int kBars = 2 * kInSlots + 4 + 2 + 5 * kOutSlots + 2;
   static constexpr int kOffTmemSlot = kOffBars + 8 * kBars;
   static constexpr int kSmemBytes = kOffTmemSlot + 8;
   static_assert(2 * kSmemBytes > 228 * 1024, "one CTA per SM: it owns all tensor memory");
@@ -93,39 +104,37 @@ struct PkParams {
   int ntiles;
 };
 
-// Quarter g (64 coefficients) of one packed row -> this thread's 16 even and
-// 16 odd operand columns.  Column order per packed word as
-// build_pack_tables' K order.
+// Quarter g (64 coefficients) of one packed row -> this thread's operand columns:
+// op[2 p + h], parity p, part h, eight words (two per 16 coefficients: x +
+// 2^(bits-1) and 2^s x of four).
 template <int kBits>
-__device__ __forceinline__ void unpack_quarter(const uint4* v, uint32_t (&ev)[16],
-                                               uint32_t (&od)[16]) {
-  if constexpr (kBits == 2) {
-    // byte_perm tables indexed by the field: x in {0, 1, -2, -1} and 64 x
-    constexpr uint32_t kX = 0xfffe0100u, kTop = 0xc0804000u;
+__device__ __forceinline__ void unpack_quarter(const uint4* v, uint32_t (&op)[4][8]) {
+  constexpr uint32_t kMask = kBits == 2 ? 0x03030303u : 0x07070707u;
+  constexpr uint32_t kSign = kBits == 2 ? 0x02020202u : 0x04040404u;
+  auto put = [&](int p, int h, int i, uint32_t w) {
+    const uint32_t f = w & kMask;
+    op[2 * p + h][2 * i] = f ^ kSign;
+    op[2 * p + h][2 * i + 1] = f << (8 - kBits);
+  };
+  auto word = [&](int i) {
+    const uint4& q = v[i >> 2];
+    return (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
+  };
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t w = i == 0 ? v[0].x : i == 1 ? v[0].y : i == 2 ? v[0].z : v[0].w;
-      const uint32_t e = w & 0x33333333u, o = (w >> 2) & 0x33333333u;
-      ev[4 * i + 0] = __byte_perm(kX, 0, e);
-      ev[4 * i + 1] = __byte_perm(kX, 0, e >> 16);
-      ev[4 * i + 2] = __byte_perm(kTop, 0, e);
-      ev[4 * i + 3] = __byte_perm(kTop, 0, e >> 16);
-      od[4 * i + 0] = __byte_perm(kX, 0, o);
-      od[4 * i + 1] = __byte_perm(kX, 0, o >> 16);
-      od[4 * i + 2] = __byte_perm(kTop, 0, o);
-      od[4 * i + 3] = __byte_perm(kTop, 0, o >> 16);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint4& q = v[i >> 2];
-      const uint32_t w = (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
-      const uint32_t e = w & 0x07070707u, o = (w >> 3) & 0x07070707u;
-      // sign-extend each byte: + 0xf8 where bit 2 is set (4 * 62 = 0xf8)
-      ev[2 * i] = e + (e & 0x04040404u) * 62u;
-      ev[2 * i + 1] = e << 5;  // 32 x: the field at the top of the byte
-      od[2 * i] = o + (o & 0x04040404u) * 62u;
-      od[2 * i + 1] = o << 5;
+  for (int i = 0; i < 4; i++) {
+    if constexpr (kBits == 2) {  // fields 0, 4, 8, 12 of a word are even j = 0, 2, 4, 6, ...
+      const uint32_t w = word(i);
+      put(0, 0, i, w);
+      put(1, 0, i, w >> 2);
+      put(0, 1, i, w >> 4);
+      put(1, 1, i, w >> 6);
+    } else {  // byte b of a word: coefficients 2 b (low field) and 2 b + 1
+      const uint32_t w0 = __byte_perm(word(2 * i), word(2 * i + 1), 0x6420);
+      const uint32_t w1 = __byte_perm(word(2 * i), word(2 * i + 1), 0x7531);
+      put(0, 0, i, w0);
+      put(1, 0, i, w0 >> 3);
+      put(0, 1, i, w1);
+      put(1, 1, i, w1 >> 3);
     }
   }
 }
@@ -163,25 +172,27 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
   constexpr uint32_t kB = 8u * (2 * S);
   auto x_ready = [&](int b) { return bars + kB + 8u * b; };
   auto op_free = [&](int b) { return bars + kB + 16u + 8u * b; };
-  auto d_full = [&](int c) { return bars + kB + 32u + 8u * c; };
-  auto d_empty = [&](int c) { return bars + kB + 48u + 8u * c; };
-  auto out_ready = [&](int b, int g) { return bars + kB + 64u + 8u * (4 * b + g); };
-  auto out_free = [&](int b) { return bars + kB + 128u + 8u * b; };
-  const uint32_t consts = bars + kB + 144u, drain = bars + kB + 152u;
+  const uint32_t d_full = bars + kB + 32u, d_empty = bars + kB + 40u;
+  auto out_ready = [&](int b, int g) { return bars + kB + 48u + 8u * (4 * b + g); };
+  constexpr int NO = L::kOutSlots;
+  auto out_free = [&](int b) { return bars + kB + 48u + 32u * NO + 8u * b; };
+  const uint32_t consts = bars + kB + 48u + 40u * NO, drain = consts + 8u;
 
   if (tid == 0) {
     for (int s = 0; s < S; s++) {
       mbar_init(in_full(s), 1);
-      mbar_init(in_empty(s), kPkEpiWarps);
+      mbar_init(in_empty(s), kPkUnpackWarps);
     }
     for (int b = 0; b < 2; b++) {
-      mbar_init(x_ready(b), kPkEpiWarps);
+      mbar_init(x_ready(b), kPkUnpackWarps);
       mbar_init(op_free(b), 2);
-      mbar_init(d_full(b), 1);
-      mbar_init(d_empty(b), 8);
+    }
+    for (int b = 0; b < NO; b++) {
       for (int g = 0; g < 4; g++) mbar_init(out_ready(b, g), 4);
       mbar_init(out_free(b), 1);
     }
+    mbar_init(d_full, 2);
+    mbar_init(d_empty, kPkEpiWarps);
     mbar_init(consts, 1);
     mbar_init(drain, 2);
     fence_mbar_init();
@@ -222,107 +233,116 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
   } else if (warp == kPkStoreWarp) {
     if (lane == 0) {
       for (int k = 0; k < nmine && ok; k++) {
-        const int b = k & 1;
+        const int b = k % NO;
         for (int g = 0; g < 4; g++) {
-          if (!(ok = mbar_wait_bounded(out_ready(b, g), (uint32_t)(k >> 1) & 1u, kPkWaitNs))) break;
+          if (!(ok = mbar_wait_bounded(out_ready(b, g), (uint32_t)(k / NO) & 1u, kPkWaitNs))) break;
           tma_store_2d(&P.out, 64 * g, kPkTile * (t_begin + k),
                        base + L::kOffOut + b * kPkOutSlot + g * kPkOutBox);
           bulk_commit();
         }
         if (!ok) break;
-        if (k >= 1) {  // tile k - 1's four boxes have been read out
-          bulk_wait_read<4>();
-          mbar_arrive(out_free(b ^ 1));
+        if (k >= NO - 1) {  // tile k - (NO - 1)'s four boxes have been read out
+          bulk_wait_read<4 * (NO - 1)>();
+          mbar_arrive(out_free((k + 1) % NO));
         }
       }
       bulk_wait_all();
     }
   } else if (warp >= kPkMmaWarp) {
     if (lane == 0) {
-      // ---- MMA issuer c: outputs 64 c .. + 63 of both parities ----
-      const int c = warp - kPkMmaWarp;
+      // ---- MMA issuer p: the coefficients of parity p ----
+      const int p = warp - kPkMmaWarp;
       // a K step's B tile: 64 rows x 32 bytes, K-major without swizzle, 2 KiB
-      const uint64_t bd = smem_desc(base + (uint32_t)c * (kPackTableBytes / 2), 128, 256,
-                                    kLayoutNone);
-      const uint32_t d = tmem + 256u + 128u * (uint32_t)c;
+      const uint64_t bd = smem_desc(base, 128, 256, kLayoutNone);
+      const uint32_t d = tmem + 256u + 128u * (uint32_t)p;
       ok = mbar_wait_bounded(consts, 0, kPkWaitNs);
       for (int k = 0; k < nmine && ok; k++) {
         const int b = k & 1;
         if (!(ok = mbar_wait_bounded(x_ready(b), (uint32_t)(k >> 1) & 1u, kPkWaitNs))) break;
-        if (k >= 1 && !(ok = mbar_wait_bounded(d_empty(c), (uint32_t)(k - 1) & 1u, kPkWaitNs)))
-          break;
+        if (k >= 1 && !(ok = mbar_wait_bounded(d_empty, (uint32_t)(k - 1) & 1u, kPkWaitNs))) break;
         tc_fence_after();
-        const uint32_t a = tmem + 128u * (uint32_t)b;
+        const uint32_t a = tmem + 128u * (uint32_t)b + 64u * (uint32_t)p;
 #pragma unroll
-        for (int par = 0; par < 2; par++)
+        for (int h = 0; h < 2; h++)
 #pragma unroll
-          for (int j = 0; j < 8; j++)
-            tc_mma_ts(d + 64u * par, a + 64u * par + 8u * j, bd + (uint64_t)(j * (2048 >> 4)),
+          for (int j = 0; j < 4; j++)
+            tc_mma_ts(d + 64u * h, a + 32u * h + 8u * j, bd + (uint64_t)((4 * h + j) * (2048 >> 4)),
                       idesc_i8(64, true, true), j != 0);
-        tc_commit(d_full(c));
+        tc_commit(d_full);
         tc_commit(op_free(b));
       }
       // every MMA issued above has completed before tensor memory is freed
       tc_commit(drain);
       ok &= mbar_wait_bounded(drain, 0, kPkWaitNs);
     }
-  } else {
-    // ---- warps 0-15: packed words -> tensor memory -> output rows ----
-    const int g = warp >> 2, lq = warp & 3, c = g >> 1;
-    const uint32_t lanes = (uint32_t)(32 * lq) << 16;
+  } else if (warp >= kPkUnpackWarp) {
+    // ---- unpack: packed words -> tensor memory, one row per thread ----
+    const int lq = warp & 3;
     const uint32_t p = (uint32_t)(32 * lq + lane);  // polynomial (row) of the tile
-    auto unpack = [&](int t) {
+    constexpr int kChunks = L::kRow / 16;
+    for (int t = 0; t < nmine; t++) {
       const int s = t % S, b = t & 1;
       bool r = mbar_wait_bounded(in_full(s), (uint32_t)(t / S) & 1u, kPkWaitNs);
       const uint32_t row = base + L::kOffIn + s * L::kInBytes + p * L::kRow;
-      uint4 v[kBits == 2 ? 1 : 2];
-      if constexpr (kBits == 2) {  // 64-byte swizzle: chunk xor (row / 2) % 4
-        v[0] = ld_shared_v4(row + (((uint32_t)g ^ ((p >> 1) & 3u)) << 4));
-      } else {  // 128-byte swizzle: chunk xor row % 8
-        v[0] = ld_shared_v4(row + (((2u * g) ^ (p & 7u)) << 4));
-        v[1] = ld_shared_v4(row + (((2u * g + 1u) ^ (p & 7u)) << 4));
-      }
+      // 64-byte rows: chunk xor (row / 2) % 4; 128-byte rows: chunk xor row % 8
+      const uint32_t x = kBits == 2 ? (p >> 1) & 3u : p & 7u;
+      uint4 v[kChunks];
+#pragma unroll
+      for (int c = 0; c < kChunks; c++) v[c] = ld_shared_v4(row + (((uint32_t)c ^ x) << 4));
       __syncwarp();
       if (lane == 0) mbar_arrive(in_empty(s));
-      uint32_t ev[16], od[16];
-      unpack_quarter<kBits>(v, ev, od);
       // the MMAs of tile t - 2 have read this operand buffer
       if (t >= 2) r &= mbar_wait_bounded(op_free(b), (uint32_t)((t >> 1) - 1) & 1u, kPkWaitNs);
-      if (!__all_sync(0xffffffffu, r)) return false;
+      if (!(ok = __all_sync(0xffffffffu, r))) break;
       tc_fence_after();
-      const uint32_t a = tmem + lanes + 128u * (uint32_t)b + 16u * (uint32_t)g;
-      tc_st16(a, ev);
-      tc_st16(a + 64u, od);
+      const uint32_t a = tmem + ((uint32_t)(32 * lq) << 16) + 128u * (uint32_t)b;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        uint32_t op[4][8];
+        unpack_quarter<kBits>(v + q * (kChunks / 4), op);
+#pragma unroll
+        for (int i = 0; i < 4; i++) tc_st8(a + 32u * i + 8u * q, op[i]);
+      }
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(x_ready(b));
-      return true;
-    };
-    if (nmine > 0) ok = unpack(0);
-    for (int k = 0; k < nmine && ok; k++) {
-      if (k + 1 < nmine && !(ok = unpack(k + 1))) break;
-      const int b = k & 1;
-      bool r = mbar_wait_bounded(d_full(c), (uint32_t)k & 1u, kPkWaitNs);
+    }
+  } else {
+    // ---- warps 0-15: sums -> output rows ----
+    const int g = warp >> 2, lq = warp & 3;
+    const uint32_t p = (uint32_t)(32 * lq + lane);  // polynomial (row) of the tile
+    const uint32_t d0 = tmem + ((uint32_t)(32 * lq) << 16) + 256u + 16u * (uint32_t)g;
+    for (int k = 0; k < nmine; k++) {
+      const int b = k % NO;
+      // the tile's sums are complete; tile k - NO's output has been read out of the slot
+      bool r = k < NO || mbar_wait_bounded(out_free(b), (uint32_t)(k / NO - 1) & 1u, kPkWaitNs);
+      r &= mbar_wait_bounded(d_full, (uint32_t)k & 1u, kPkWaitNs);
       if (!(ok = __all_sync(0xffffffffu, r))) break;
       tc_fence_after();
-      uint32_t s[64];  // outputs 32 g .. + 31 of each parity
-      const uint32_t d = tmem + lanes + 256u + 128u * (uint32_t)c + 32u * (uint32_t)(g & 1);
-      tc_ld32x2_sync(d, d + 64u, s);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(d_empty(c));
-      // tile k - 2's output has been read out of this slot
-      r = k < 2 || mbar_wait_bounded(out_free(b), (uint32_t)((k >> 1) - 1) & 1u, kPkWaitNs);
-      if (!(ok = __all_sync(0xffffffffu, r))) break;
       const uint32_t row = base + L::kOffOut + b * kPkOutSlot + g * kPkOutBox + p * 128u;
 #pragma unroll
-      for (int j = 0; j < 8; j++)
-        st_shared_v4(row + (((uint32_t)j ^ (p & 7u)) << 4),
-                     reduce_pair(s[4 * j], s[32 + 4 * j]),
-                     reduce_pair(s[4 * j + 1], s[32 + 4 * j + 1]),
-                     reduce_pair(s[4 * j + 2], s[32 + 4 * j + 2]),
-                     reduce_pair(s[4 * j + 3], s[32 + 4 * j + 3]));
+      for (int h = 0; h < 2; h++) {
+        uint32_t s[32];  // rows 16 g + 8 h .. + 7: even P, even M, odd P, odd M
+        const uint32_t d = d0 + 8u * h;
+        tc_ld8x4_sync(d, d + 64u, d + 128u, d + 192u, s);
+        if (h == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(d_empty);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          uint32_t w[4];  // rows 2 j and 2 j + 1: two output pairs each
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int m = 2 * j + i;
+            w[2 * i] = reduce_pair(s[m] + s[8 + m], s[16 + m] + s[24 + m]);
+            w[2 * i + 1] = reduce_pair(s[m] - s[8 + m], s[16 + m] - s[24 + m]);
+          }
+          st_shared_v4(row + (((uint32_t)(4 * h + j) ^ (p & 7u)) << 4), w[0], w[1], w[2], w[3]);
+        }
+      }
       fence_proxy_async_smem();  // generic-proxy writes -> the TMA store
       __syncwarp();
       if (lane == 0) mbar_arrive(out_ready(b, g));

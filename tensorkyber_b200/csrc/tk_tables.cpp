@@ -4,6 +4,7 @@
 // them into 7-bit INT8 limb fragments in mma.sync register order.
 #include "tk_tables.h"
 
+#include <stdlib.h>
 #include <string.h>
 
 namespace tk {
@@ -295,7 +296,7 @@ void build_tc5_tables(const Matrices& M, uint8_t* out) {
 }
 
 void build_pack_tables(int bits, uint8_t* out) {
-  const int s = 8 - bits;
+  const int s = 8 - bits, unit = 1 << s;
   int64_t v[256];
   int16_t F[128][128];
   for (int j = 0; j < 128; j++) {
@@ -305,13 +306,41 @@ void build_pack_tables(int bits, uint8_t* out) {
     for (int t = 0; t < 128; t++)
       F[t][j] = (int16_t)(v[2 * t] > (kQ - 1) / 2 ? v[2 * t] - kQ : v[2 * t]);
   }
-  for (int t = 0; t < 128; t++)
-    for (int k = 0; k < 256; k++) {
-      const PackPos at = pack_k_pos(bits, k);
-      const int c = F[t][at.j], half = 1 << (s - 1);
-      const int c0 = ((c + half) & ((1 << s) - 1)) - half, c1 = (c - c0) >> s;
-      out[2048 * (8 * (t >> 6) + (k >> 5)) + tc5_tile_offset(t & 63, k & 31)] =
-          (uint8_t)(int8_t)(at.top ? c1 : c0);
+  for (int h = 0; h < 2; h++)
+    for (int m = 0; m < 64; m++) {
+      // row 2m over j = 2i + h: c0 in [-unit/2, unit/2), c1 = (c - c0) / unit
+      int c[64], c0[64], sum = 0;
+      auto split = [&](int i) { c0[i] = ((c[i] + unit / 2) & (unit - 1)) - unit / 2; };
+      for (int i = 0; i < 64; i++) {
+        c[i] = F[2 * m][2 * i + h];
+        split(i);
+        sum += c0[i];
+      }
+      // the sum of the c0 to zero: q = 1 mod unit, so c -+ q moves one c0 by -+ 1 (the
+      // constants that end up smallest first) ...
+      while (sum & (unit - 1)) {
+        const int d = (sum & (unit - 1)) <= unit / 2 ? -1 : 1;  // direction of the c0
+        int best = -1;
+        for (int i = 0; i < 64; i++)
+          if (best < 0 || abs(c[i] + d * kQ) < abs(c[best] + d * kQ)) best = i;
+        sum -= c0[best];
+        c[best] += d * kQ;
+        split(best);
+        sum += c0[best];
+      }
+      // ... then c0 +- unit with c1 -+ 1, one constant after the other
+      for (int i = 0; sum != 0; i = (i + 1) & 63) {
+        const int d = sum > 0 ? -unit : unit;
+        if (c0[i] + d < -128 || c0[i] + d > 127) continue;
+        c0[i] += d;
+        sum += d;
+      }
+      for (int k = 0; k < 128; k++) {
+        const PackPos at = pack_k_pos(h, k);
+        const int i = at.j >> 1;
+        out[2048 * (4 * h + (k >> 5)) + tc5_tile_offset(m, k & 31)] =
+            (uint8_t)(int8_t)(at.top ? (c[i] - c0[i]) / unit : c0[i]);
+      }
     }
 }
 

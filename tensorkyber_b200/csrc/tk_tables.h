@@ -161,23 +161,24 @@ inline int tc5_tile_offset(int n, int k) {
 }
 void build_tc5_tables(const Matrices& M, uint8_t* out /* kTc5TableBytes */);
 
-// B operand of the dense packed forward (tk_pack.cu) for bits = 2 or 3: the
-// 128 x 128 matrix F of either parity (out[2t + p] = sum_j F[t][j] x[2j + p]),
-// each constant centred and split as c0 + 2^s c1, s = 8 - bits, both int8.
-// Output half h (t = 64 h + n), K step i (32 of the 256 K bytes): a tile of 64
-// rows x 32 bytes at 2048 (8 h + i), laid out as tc5_tile_offset(n, k).
-// pack_k_pos says what K byte k of a row is: coefficient j of the parity, as x
-// (constant c0) or moved up by s bits (constant c1).
-constexpr int kPackTableBytes = 2 * 8 * 2048;
+// B operand of the dense packed forward (tk_pack.cu) for bits = 2 or 3.  Either
+// parity meets the matrix F (out[2t + p] = sum_j F[t][j] x[2j + p]) whose rows 2m
+// and 2m + 1 belong to roots z and -z: with P_m and M_m the sums of row 2m over
+// even and odd j, the two outputs are P_m + M_m and P_m - M_m.  Part h (0: P, 1:
+// M), K step i (32 of its 128 K bytes): a tile of 64 rows m x 32 bytes at 2048 (4
+// h + i), laid out as tc5_tile_offset(m, k).  Each constant is taken mod q as c0 +
+// 2^s c1, s = 8 - bits, both int8: the data carry x + 2^(bits-1) (constant c0) and
+// 2^s x (constant c1), and the c0 of a row sum to zero, so the offset drops out.
+// pack_k_pos says what K byte k of a part is: coefficient j of the parity, as x +
+// 2^(bits-1) or (top) moved up by s bits.
+constexpr int kPackTableBytes = 2 * 4 * 2048;
 struct PackPos {
   int j;
   bool top;
 };
-inline PackPos pack_k_pos(int bits, int k) {
-  const int col = k >> 2, b = k & 3;
-  if (bits == 2)  // four words per packed word: x of its 8 coefficients, then 64 x
-    return PackPos{8 * (col >> 2) + 4 * (col & 1) + b, (col & 2) != 0};
-  return PackPos{4 * (col >> 1) + b, (col & 1) != 0};  // two per word: x, 32 x
+inline PackPos pack_k_pos(int h, int k) {
+  const int col = k >> 2;  // operand word: pairs (x + offset, 2^s x) of four coefficients
+  return PackPos{8 * (col >> 1) + 2 * (k & 3) + h, (col & 1) != 0};
 }
 void build_pack_tables(int bits, uint8_t* out /* kPackTableBytes */);
 

@@ -47,42 +47,52 @@ def reduce_pair(s0, s1):
 
 
 def test_reduce_pair_is_exact_over_its_range():
-    s = np.arange(-128 * 4 * 1664, 128 * 4 * 1664 + 1, dtype=np.int64)
+    s = np.arange(-(1 << 20), (1 << 20) + 1, dtype=np.int64)
     for other in (s[::-1], np.full_like(s, s[0]), np.full_like(s, s[-1])):
         assert (reduce_pair(s, other) == (s % Q) + ((other % Q) << 16)).all()
         assert (reduce_pair(other, s) == (other % Q) + ((s % Q) << 16)).all()
 
 
 def operand(bits, packed):
-    """The even and odd operand rows (signed bytes, [n][256]) of packed rows."""
+    """The operand rows (signed bytes, [n][128]) of packed rows, [parity][part]."""
     w = packed.reshape(packed.shape[0], -1).view(np.uint32)
+    mask, sign = (0x03030303, 0x02020202) if bits == 2 else (0x07070707, 0x04040404)
+    if bits == 2:
+        fields = [[w, w >> np.uint32(4)], [w >> np.uint32(2), w >> np.uint32(6)]]
+    else:
+        by = packed.reshape(packed.shape[0], -1, 8)           # bytes of a word pair
+        halves = [np.ascontiguousarray(by[:, :, h::2]).view(np.uint32)[..., 0] for h in (0, 1)]
+        fields = [halves, [v >> np.uint32(3) for v in halves]]
     out = []
-    for parity in (0, 1):
-        if bits == 2:
-            f = (w >> np.uint32(2 * parity)) & np.uint32(0x33333333)
-            x, top = np.array([0, 1, -2, -1], np.int8), np.array([0, 64, -128, -64], np.int8)
-            nib = np.stack([(f >> np.uint32(4 * i)) & np.uint32(3) for i in range(8)], axis=2)
-            row = np.concatenate([x[nib], top[nib]], axis=2)        # [n][word][16]
-        else:
-            f = (w >> np.uint32(3 * parity)) & np.uint32(0x07070707)
-            x = f + (f & np.uint32(0x04040404)) * np.uint32(62)
-            row = np.stack([x, f << np.uint32(5)], axis=2).view(np.int8)
-        out.append(row.reshape(w.shape[0], 256).astype(np.int64))
+    for per_part in fields:
+        out.append([])
+        for f in per_part:
+            f = f & np.uint32(mask)
+            row = np.stack([f ^ np.uint32(sign), f << np.uint32(8 - bits)], axis=2)
+            out[-1].append(row.view(np.int8).reshape(w.shape[0], 128).astype(np.int64))
     return out
 
 
 @pytest.mark.parametrize("bits,lo,hi", [(2, -2, 1), (3, -4, 3)])
 def test_packed_forward_model(table, oracle, bits, lo, hi):
-    raw = table(f"build_pack_tables({bits}, out);", 2 * 8 * 2048)
-    B = np.concatenate([np.concatenate([decode(raw[2048 * (8 * h + i):][:2048], 64)
-                                        for i in range(8)], axis=1) for h in (0, 1)])
-    B = B.view(np.int8).astype(np.int64)                               # [128 outputs][256]
+    raw = table(f"build_pack_tables({bits}, out);", 2 * 4 * 2048)
+    B = [np.concatenate([decode(raw[2048 * (4 * h + i):][:2048], 64) for i in range(4)],
+                        axis=1).view(np.int8).astype(np.int64) for h in (0, 1)]
+    for b in B:                            # words alternate: constants of x - lo, of 2^s x
+        c0, c1 = b.reshape(64, 32, 4)[:, 0::2], b.reshape(64, 32, 4)[:, 1::2]
+        assert (c0.sum((1, 2)) == 0).all()                     # the offset drops out
+    # |P +- M| over every input: the reduction's exact range
+    worst = sum(np.abs(b.reshape(64, 32, 4)[:, 0::2] + (1 << (8 - bits)) *
+                       b.reshape(64, 32, 4)[:, 1::2]).sum((1, 2)) for b in B) * -lo
+    assert worst.max() < 1 << 20
     r = rng(bits)
     x = r.integers(lo, hi + 1, size=(96, 256)).astype(np.int16)
     x[0], x[1] = lo, hi
-    ev, od = operand(bits, oracle.pack_small(bits, x))
-    s0, s1 = ev @ B.T, od @ B.T
-    assert max(np.abs(s0).max(), np.abs(s1).max()) <= 128 * -lo * 1664
-    pair = reduce_pair(s0, s1)
-    got = np.stack([pair & 0xffff, pair >> 16], axis=2).reshape(-1, 256)
+    sums = [[part @ b.T for part, b in zip(parts, B)]
+            for parts in operand(bits, oracle.pack_small(bits, x))]
+    got = np.zeros((96, 256), dtype=np.int64)
+    for sign, at in ((1, 0), (-1, 2)):
+        s0, s1 = (p + sign * m for p, m in sums)
+        pair = reduce_pair(s0, s1)
+        got[:, at::4], got[:, at + 1::4] = pair & 0xffff, pair >> 16
     assert (got == canon(oracle.ntt(x))).all()
