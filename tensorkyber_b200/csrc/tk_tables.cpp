@@ -266,7 +266,7 @@ void build_tile_frags(const Matrices& M, TileFrags* F) {
           F->sa[b][s]);
 }
 
-void build_tc5_tables(const Matrices& M, uint8_t* out) {
+void build_tc5_tables(const Matrices& M, uint8_t* out, bool signed_sums) {
   memset(out, 0, kTc5TableBytes);
   auto put = [&](int tile, int n, int k, int64_t v) {
     out[tile * kTc5TileBytes + tc5_tile_offset(n, k)] = (uint8_t)v;
@@ -284,14 +284,19 @@ void build_tc5_tables(const Matrices& M, uint8_t* out) {
           put(34 + b, o + 16 * g, 2 * j + b, limb(byte_weighted(M.m1[o][j], b), g));
         }
   // second stages: four bytes of an int32 sum per input, two K steps of 8
+  const int64_t kInv255 = 1188;  // 255^-1 mod q
+  auto sum_byte = [&](int64_t c, int t) {
+    const int64_t v = byte_weighted(c, t);
+    return signed_sums && t == 3 ? modq(-v * kInv255) : v;
+  };
   for (int o = 0; o < 16; o++)
     for (int g = 0; g < 2; g++)
       for (int j = 0; j < 16; j++)
         for (int t = 0; t < 4; t++) {
           const int h = j >> 3, k = 4 * (j & 7) + t;
-          put(32 + h, o + 16 * g, k, limb(byte_weighted(M.minv[o][j], t), g));
+          put(32 + h, o + 16 * g, k, limb(sum_byte(M.minv[o][j], t), g));
           for (int i = 0; i < 16; i++)
-            put(36 + 2 * i + h, o + 16 * g, k, limb(byte_weighted(M.m2[i][o][j], t), g));
+            put(36 + 2 * i + h, o + 16 * g, k, limb(sum_byte(M.m2[i][o][j], t), g));
         }
 }
 

@@ -159,7 +159,13 @@ constexpr int kTc5TableBytes = kTc5Tiles * kTc5TileBytes;
 inline int tc5_tile_offset(int n, int k) {
   return (n >> 3) * 256 + (k >> 4) * 128 + (n & 7) * 16 + (k & 15);
 }
-void build_tc5_tables(const Matrices& M, uint8_t* out /* kTc5TableBytes */);
+// signed_sums (the kernels' own tiles): the first-stage sums come as they are,
+// signed, below 2^24 in magnitude (at most 5.1 M in the inverse, 11.2 M in the
+// forward), so their top byte, read as unsigned, is 0 or 255, and its constant is
+// -2^24 C / 255 mod q.  Without it the top byte carries 256^3 C, for sums made
+// non-negative by a bias.
+void build_tc5_tables(const Matrices& M, uint8_t* out /* kTc5TableBytes */,
+                      bool signed_sums = false);
 
 // B operand of the dense packed forward (tk_pack.cu) for bits = 2 or 3.  Either
 // parity meets the matrix F (out[2t + p] = sum_j F[t][j] x[2j + p]) whose rows 2m

@@ -23,12 +23,14 @@
 //     constants on the low bytes' K rows, one with signed data and constants
 //     256 C mod q on the high bytes' K rows; the other rows of each constant
 //     tile are zero.
-//   * The first stage's sums S = D_lo + 128 D_hi are never reduced: S + 2048 q
-//     (non-negative, below 2^25) goes back to tensor memory as int32,
-//     transposed -- output n's second-stage operand is the 16 columns 16 n ..
-//     16 n + 15, read by tcgen05.mma straight from tensor memory as 64
-//     unsigned bytes whose constants carry 256^j mod q, two MMAs per
-//     coefficient (inverse) or block (forward).
+//   * The first stage's sums S = D_lo + 128 D_hi are never reduced: they go back
+//     to tensor memory as int32, transposed -- output n's second-stage operand
+//     is the 16 columns 16 n .. 16 n + 15, read by tcgen05.mma straight from
+//     tensor memory as 64 unsigned bytes, two MMAs per coefficient (inverse) or
+//     block (forward).  Bytes 0-2 meet constants times 256^j mod q.  |S| < 2^24,
+//     so the top byte is 0 or 255 (the sign), and its constant is -2^24 C / 255:
+//     no bias is added to make the sums non-negative (one instruction of 12 per
+//     coefficient).
 //   * The second stage's sums (below 2^26) get one exact reduction (centred
 //     for the inverse, [0, q) for the forward), are packed to int16 and
 //     written in the TMA layout over the tile's own input slot (its MMAs have
@@ -114,11 +116,6 @@ constexpr uint32_t kColD0 = 256;  // group g's accumulator buffer at kColD0 + 64
 constexpr uint32_t kIdescU8 = idesc_i8(32, false, false);
 constexpr uint32_t kIdescS8 = idesc_i8(32, true, true);
 constexpr uint64_t kWaitNs = 2000000000ull;
-// The first stage's sums S (in [-16 * 128 (q-1), 16 * 382 (q-1)]: unsigned
-// low bytes and signed high bytes against constants below q) plus this
-// multiple of q are non-negative and below 2^25: bytes 0-2 and a top byte of
-// 0 or 1, all unsigned for the second stage.
-constexpr uint32_t kFirstBias = 2048u * 3329u;
 
 __device__ __align__(128) uint8_t g_tc5_tables[kTc5TableBytes];
 
@@ -419,8 +416,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
         ok = false;
         break;
       }
-      // first stage: S = D_lo + 128 D_hi + 2048 q (non-negative, below 2^25)
-      // as int32 to tensor memory column 16 n + idx (output n of result idx),
+      // first stage: S = D_lo + 128 D_hi (signed, below 2^24 in magnitude) as
+      // int32 to tensor memory column 16 n + idx (output n of result idx),
       // the second stage's K bytes 4 (idx % 8) .. + 3 of step idx / 8.  The
       // previous tile's second-stage MMAs (from every issuer) read these
       // columns: y_free says they have finished.
@@ -439,8 +436,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
         give_back();
 #pragma unroll
         for (int n = 0; n < 16; n++)
-          tc_st2(ycol + 16u * n + 2u * a, r[n] + (r[16 + n] << 7) + kFirstBias,
-                 r[32 + n] + (r[48 + n] << 7) + kFirstBias);
+          tc_st2(ycol + 16u * n + 2u * a, r[n] + (r[16 + n] << 7),
+                 r[32 + n] + (r[48 + n] << 7));
         if (jj == 0) {
           // the sums of first-stage chunks 0-3 (columns 16 n .. 16 n + 7,
           // the second stage's K step 0) are written once all 16 warps arrive
@@ -581,7 +578,7 @@ bool tc5_init_device(DeviceInfo* info) {
   std::call_once(once, [] {
     static Matrices M;
     build_matrices(&M);
-    build_tc5_tables(M, image);
+    build_tc5_tables(M, image, true);
   });
   if (info->device < 0 || info->device >= 64) return false;
   if (cudaMemcpyToSymbol(g_tc5_tables, image, sizeof(image)) != cudaSuccess) return false;

@@ -96,3 +96,42 @@ def test_packed_forward_model(table, oracle, bits, lo, hi):
         pair = reduce_pair(s0, s1)
         got[:, at::4], got[:, at + 1::4] = pair & 0xffff, pair >> 16
     assert (got == canon(oracle.ntt(x))).all()
+
+
+def test_tc5_signed_first_stage_sums(table, oracle):
+    """The tcgen05 inverse and forward on signed first-stage sums: below 2^24 for
+    every input, their top byte (0 or 255) weighted by the kernels' own tiles."""
+    from test_tc5_model import as_s8, as_u8, decode as decode_tiles
+    t = decode_tiles(table("static Matrices M; build_matrices(&M); build_tc5_tables(M, out, true);",
+                           68 * 1024))
+    x = rng(77).integers(-32768, 32768, size=(64, 256)).astype(np.int16)
+    x[0], x[1], x[2] = -32768, 32767, np.where(np.arange(256) % 2, -32768, 32767)
+    raw = x.view(np.uint8).reshape(64, 256, 2)
+
+    def first(by, lo, hi):
+        d = as_u8(by) @ lo.T + as_s8(by) @ hi.T
+        return d[:, :16] + 128 * d[:, 16:]
+
+    def second(s, tiles):
+        by = np.ascontiguousarray(s.astype(np.int32)).view(np.uint8).reshape(-1, 64).astype(np.int64)
+        d = by[:, :32] @ tiles[0].T + by[:, 32:] @ tiles[1].T
+        v = d[:, :16] + 128 * d[:, 16:]
+        assert v.min() >= 0 and v.max() + 1664 < 1 << 26
+        return v % Q
+    # the bound of the sums over all inputs: low bytes 0..255, high bytes -128..127
+    for lo, hi in [(t[2 * m], t[2 * m + 1]) for m in range(16)] + [(t[34], t[35])]:
+        top = (255 * lo.sum(1) + 127 * hi.sum(1)).reshape(2, 16)
+        low = (-128 * hi.sum(1)).reshape(2, 16)
+        assert (top[0] + 128 * top[1]).max() < 1 << 24 and (low[0] + 128 * low[1]).min() > -(1 << 24)
+    inv = np.zeros((64, 16, 16), dtype=np.int64)
+    Y = np.stack([first(raw[:, 16 * m:16 * m + 16].reshape(64, 32), t[2 * m], t[2 * m + 1])
+                  for m in range(16)], axis=1)                        # [p][m][c]
+    fwd = np.zeros((64, 16, 16), dtype=np.int64)
+    Z = np.stack([first(np.ascontiguousarray(raw.reshape(64, 16, 16, 2)[:, :, c]).reshape(64, 32),
+                        t[34], t[35]) for c in range(16)], axis=2)    # [p][i][c]
+    for n in range(16):
+        inv[:, :, n] = second(Y[:, :, n], t[32:34])
+        fwd[:, n] = second(Z[:, n], t[36 + 2 * n:38 + 2 * n])
+    c = canon(x).astype(np.int16)
+    assert (inv.reshape(64, 256) == canon(oracle.invntt(c))).all()
+    assert (fwd.reshape(64, 256) == canon(oracle.ntt(c))).all()
