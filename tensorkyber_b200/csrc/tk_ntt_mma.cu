@@ -791,8 +791,9 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
 // Tiles are numbered across the batches (batch b owns [first_tile[b],
 // first_tile[b+1])) and CTA c takes tiles c, c + G, c + 2G, ... (G CTAs), so
 // the launch has one tail for all batches and its CTAs run one k at a time.
-// Two slots: the next tile's s loads into the other one once the store of the
-// tile before has been read out of it.  Rows past a batch are out of
+// One slot: the next tile's s loads into it once this tile's store has been read
+// out (the SM's other three CTAs cover the wait), which leaves room for the
+// forward's unreduced int32 sums.  Rows past a batch are out of
 // bounds of its tensor maps (zero-filled in; boxes that start past it are
 // neither loaded nor stored) and jobs past it are skipped.  The stage
 // constants are re-read from L1 at each stage, so that between stages their
@@ -808,7 +809,10 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
 // 129.4 us; in a seconds-long loop, where the 1 kW limit holds the clock and
 // energy counts, 140.1 -> 136.2.  A 24-row tile's polynomial stages on all four
 // warps, six rows each, instead of eight on three: k = 3 alone 70.2 -> 66.4 us,
-// the mix 129.6 -> 126.3.  Five or six CTAs per SM at 96 or 80 registers:
+// the mix 129.6 -> 126.3.  The forward on int32 sums as the batch kernel's variant
+// 3 (20 instructions per polynomial fewer), in the room of the second slot: 125.5
+// -> 121.8 us, 16,383 jobs 36.8 -> 36.0 (in a long loop 39.9 -> 37.5), 37 jobs of k
+// = 4 6.7 -> 6.4; with both slots kept, three CTAs per SM, 129 us.  Five or six CTAs per SM at 96 or 80 registers:
 // 133.2 / 132.6 us.
 struct MvTiles {
   CUtensorMap s_map[kMaxSegs];    // s rows [njobs * k][128 words], 8 x 132-word boxes
@@ -829,7 +833,8 @@ __device__ TileFrags g_tile_sa;
 __device__ InvFrags g_tile_inv;
 
 constexpr int kTileSlotBytes = 32 * kRowBytes;      // one 32-row slot
-constexpr int kTileSmem = 2 * kTileSlotBytes + 16;  // two tile slots, 2 mbarriers
+constexpr int kTileWideBytes = 32 * kWideRowBytes;  // the forward's int32 sums
+constexpr int kTileSmem = kTileSlotBytes + kTileWideBytes + 16;  // and an mbarrier
 __host__ __device__ constexpr int tile_units(int k) { return k == 3 ? 3 : 4; }
 __host__ __device__ constexpr int tile_jobs(int k) { return 8 * tile_units(k) / k; }
 
@@ -844,8 +849,11 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   // (one k's code at a time)
   const int G = (int)gridDim.x;
   const int nmine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / G + 1 : 0;
-  const uint32_t smem0 = smem_u32(smem);
-  const uint32_t bar0 = smem0 + 2 * kTileSlotBytes;
+  const uint32_t slot = smem_u32(smem);
+  uint8_t* const slotp = smem;
+  const uint32_t inter = slot + kTileSlotBytes;
+  uint8_t* const interp = smem + kTileSlotBytes;
+  const uint32_t bar0 = inter + kTileWideBytes;
 
   const int blk0 = 4 * warp;
   int32_t zc[PP][2][2];
@@ -883,7 +891,6 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
 
   if (tid == 0) {
     mbar_init(bar0, W);
-    mbar_init(bar0 + 8, W);
     fence_mbar_init();
   }
   __syncthreads();
@@ -893,11 +900,18 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
 
   const int q4 = lane & 3, g8 = lane >> 2;
   const uint32_t ldt_off = 32u * ((lane & 7) + 8 * ((lane >> 3) & 1)) + 16u * (lane >> 4);
-  const uint32_t hb1 = (lane >> 4) & 1;
-  const uint32_t w_even = 32u * g8 + 16u * hb1 + 4u * q4;
-  const uint32_t w_odd = 32u * g8 + 16u * (hb1 ^ 1) + 4u * q4;
   const uint32_t w_nat = 32u * g8 + 4u * q4;
   const uint32_t hbw = (uint32_t)((blk0 >> 2) & 1);
+  const uint32_t swz1 = (uint32_t)(g8 >> 1) & 1u;
+  const uint32_t wi_e = 64u * g8 + 32u * swz1 + 8u * q4;
+  const uint32_t wi_o = 64u * g8 + 32u * (swz1 ^ 1u) + 8u * q4;
+  uint32_t ldw[PP];
+#pragma unroll
+  for (int p = 0; p < PP; p++) {
+    const int I = blk0 + 2 * p;
+    const uint32_t par = ((uint32_t)(lane >> 4) & 1u) ^ ((uint32_t)(I >> 1) & 1u);
+    ldw[p] = kWideRowBytes * (lane & 7) + 64u * I + 32u * par + 16u * ((lane >> 3) & 1);
+  }
   const uint32_t ldc_base = kRowBytes * (lane & 7) + 32u * (lane >> 4);
   const uint32_t ldc_split = ldc_base + 16u * (((lane >> 3) & 1) ^ hbw);
   const uint32_t stc_off = kRowBytes * (2 * q4) + 4u * g8;
@@ -919,17 +933,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     for (int j = 1; j < kMaxSegs; j++) b += (j < P.nb && t >= P.first_tile[j]);
     return b;
   };
-  auto issue_load = [&](int k, int slot_i) {
+  auto issue_load = [&](int k) {
     if (lane != 0) return;
-    const uint32_t bar = bar0 + 8 * slot_i;
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), kb = P.k[b];
     const int row = (t - P.first_tile[b]) * 8 * tile_units(kb) + 8 * warp;
     if (warp < tile_units(kb) && row < P.njobs[b] * kb) {  // boxes past the batch: none
-      mbar_expect_tx(bar, kWarpBoxBytes);
-      tma_load_2d(smem0 + slot_i * kTileSlotBytes + warp * kWarpBoxBytes, &P.s_map[b], 0, row,
-                  bar);
+      mbar_expect_tx(bar0, kWarpBoxBytes);
+      tma_load_2d(slot + warp * kWarpBoxBytes, &P.s_map[b], 0, row, bar0);
     } else {
-      mbar_expect_tx(bar, 0);  // arrive only
+      mbar_expect_tx(bar0, 0);  // arrive only
     }
   };
   // A and e of tile k into L2 (one thread; the ranges stop at the batch end),
@@ -947,27 +959,36 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
 
   // A tile's three phases.  The NTT phases depend on the tile's unit count
   // only (4 for k = 2, 4; 3 for k = 3), so k = 2 and k = 4 share their code.
-  // forward NTT of the s tile (in the given slot), in place
-  auto fwd_phase = [&](auto nc, uint32_t slot, uint8_t* slotp) {
+  // forward NTT of the s tile, by way of the int32 sums, back into the slot
+  auto fwd_phase = [&](auto nc) {
     constexpr int NU = decltype(nc)::value;
     {
       uint32_t fam[2][4];
       load_am(g_fwd.s1, fam);
       const uint2 c1 = ldg_keep_u2(&g_fwd.c1[lane][0]);
-      const int32_t cbz[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
       constexpr int kR = 2 * NU;  // rows per warp
-      poly_stage<false, false, kR>(slot + kR * warp * kRowBytes, slotp + kR * warp * kRowBytes,
-                                   ldt_off, fam, (int32_t)c1.x, (int32_t)c1.y, cbz, w_even, w_odd,
-                                   0, nullptr, 0, 0, 0);
+      poly_stage_fwd_wide<kR>(slot + kR * warp * kRowBytes, interp + kR * warp * kWideRowBytes,
+                              ldt_off, fam, (int32_t)c1.x, (int32_t)c1.y, wi_e, wi_o);
     }
     cta_sync_named();
-    uint32_t fac[PP][2][2][2];
-    load_ac(g_fwd.s2, fac);
-    block_stage<true, true, W, PP, NU>(slot, slotp, blk0, ldc_split, stc_off, fac, zc);
+    uint32_t fac[PP][2][2][4];
+#pragma unroll
+    for (int p = 0; p < PP; p++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+          const uint4 v = ldg_keep_u4(&g_fwd.s2w[blk0 + 2 * p + h][s][lane][0]);
+          fac[p][h][s][0] = v.x;
+          fac[p][h][s][1] = v.y;
+          fac[p][h][s][2] = v.z;
+          fac[p][h][s][3] = v.w;
+        }
+    block_stage_wide<NU>(inter, slotp, blk0, ldw, stc_off, fac);
   };
   // basemul-accumulate in place, one job per warp at a time, its loads of A
   // issued first (k = 4: half of them, which leaves registers and loses no time)
-  auto basemul_phase = [&](auto kc, int b, int tl, uint8_t* slotp) {
+  auto basemul_phase = [&](auto kc, int b, int tl) {
     constexpr int K = decltype(kc)::value;
     constexpr int kJobs = tile_jobs(K);
     const int njobs = P.njobs[b];
@@ -1005,12 +1026,12 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     }
   };
   // inverse NTT plus e on the accumulators, in place; then the store
-  auto inv_phase = [&](auto nc, uint32_t acc, uint8_t* accp, int b, int row0, int nvec) {
+  auto inv_phase = [&](auto nc, int b, int row0, int nvec) {
     constexpr int NU = decltype(nc)::value;
     {
       uint32_t iac[PP][2][2][2];
       load_ac(g_tile_sa.sa, iac);
-      block_stage<true, true, W, PP, NU>(acc, accp, blk0, ldc_split, stc_inv, iac, zc);
+      block_stage<true, true, W, PP, NU>(slot, slotp, blk0, ldc_split, stc_inv, iac, zc);
     }
     cta_sync_named();
     constexpr int kR = 2 * NU;  // rows per warp
@@ -1018,7 +1039,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     load_am(g_tile_inv.sb, iam);
     const int32_t cbz[2][4] = {{kCentre, kCentre, kCentre, kCentre},
                                {kCentre, kCentre, kCentre, kCentre}};
-    poly_stage<true, true, kR>(acc + kR * warp * kRowBytes, accp + kR * warp * kRowBytes, ldt_inv,
+    poly_stage<true, true, kR>(slot + kR * warp * kRowBytes, slotp + kR * warp * kRowBytes, ldt_inv,
                                iam, 0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + kR * warp, nvec,
                                8u * g8 + q4);
     fence_proxy_async_smem();
@@ -1027,18 +1048,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     else
       cta_sync_named();  // a box's rows come from two warps
     if (lane == 0 && warp < NU && row0 + 8 * warp < nvec)  // boxes past the batch are dropped
-      tma_store_2d(&P.out_map[b], 0, row0 + 8 * warp, acc + warp * kWarpBoxBytes);
+      tma_store_2d(&P.out_map[b], 0, row0 + 8 * warp, slot + warp * kWarpBoxBytes);
     if (lane == 0) bulk_commit();  // every lane-0 keeps one (possibly empty) group per tile
   };
   using U3 = std::integral_constant<int, 3>;
   using U4 = std::integral_constant<int, 4>;
 
-  issue_load(0, 0);
+  issue_load(0);
   for (int k = 0; k < nmine; k++) {
-    const int slot_i = k & 1;
-    const uint32_t slot = smem0 + slot_i * kTileSlotBytes;
-    uint8_t* const slotp = smem + slot_i * kTileSlotBytes;
-    const bool ok = mbar_wait_bounded(bar0 + 8 * slot_i, (uint32_t)(k >> 1) & 1u, kWaitLimitNs);
+    const bool ok = mbar_wait_bounded(bar0, (uint32_t)k & 1u, kWaitLimitNs);
     if (!__syncthreads_and(ok)) {  // CTA-uniform give-up
       if (tid == 0) atomicOr(&g_status, 16u);
       break;
@@ -1048,25 +1066,24 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     const int kb = P.k[b];  // CTA-uniform
     const int row0 = tl * 8 * tile_units(kb), nvec = P.njobs[b] * kb;
     if (tile_units(kb) == 3)  // the phase code for the tile's unit count
-      fwd_phase(U3{}, slot, slotp);
+      fwd_phase(U3{});
     else
-      fwd_phase(U4{}, slot, slotp);
-    if (k + 1 < nmine) {
-      // the other slot held tile k-1: its store (this lane's own box) has been read out
-      if (lane == 0) bulk_wait_read<0>();
-      issue_load(k + 1, slot_i ^ 1);
-    }
+      fwd_phase(U4{});
     cta_sync_named();
     switch (kb) {
-      case 2: basemul_phase(std::integral_constant<int, 2>{}, b, tl, slotp); break;
-      case 3: basemul_phase(std::integral_constant<int, 3>{}, b, tl, slotp); break;
-      default: basemul_phase(std::integral_constant<int, 4>{}, b, tl, slotp); break;
+      case 2: basemul_phase(std::integral_constant<int, 2>{}, b, tl); break;
+      case 3: basemul_phase(std::integral_constant<int, 3>{}, b, tl); break;
+      default: basemul_phase(std::integral_constant<int, 4>{}, b, tl); break;
     }
     cta_sync_named();
     if (tile_units(kb) == 3)  // the phase code for the tile's unit count
-      inv_phase(U3{}, slot, slotp, b, row0, nvec);
+      inv_phase(U3{}, b, row0, nvec);
     else
-      inv_phase(U4{}, slot, slotp, b, row0, nvec);
+      inv_phase(U4{}, b, row0, nvec);
+    if (k + 1 < nmine) {
+      if (lane == 0) bulk_wait_read<0>();  // this lane's own box
+      issue_load(k + 1);
+    }
   }
   if (lane == 0) bulk_wait_all();
 }
