@@ -62,6 +62,17 @@
 namespace tk {
 
 constexpr int kWarpBoxBytes = 8 * kRowBytes;      // one TMA box: 8 padded rows
+// The forward's input on wide kernels, whose first stage writes elsewhere: each
+// polynomial as four quarters of 128 bytes (4 blocks) 144 bytes apart.  The first
+// stage's ldmatrix.trans takes the same 16-byte half of eight blocks: 32 bytes
+// apart, as in a padded row, two of them share each bank group; with the pad
+// after every quarter none do.  Eight polynomials (a TMA box) take 4,608 bytes, and
+// the 8 padded output rows of the same unit go to the same place.  40,009
+// polynomials 10.5 -> 10.2 us, 262,144 47.0 -> 46.3, 2^20 182 -> 173 (in a long loop
+// at the power limit 198 -> 193).  TMA's 32-byte swizzle gives the same banks, but
+// its 32-byte pieces load slower: 262,144 49.4 us.
+constexpr int kSplitRowBytes = 4 * 144;
+constexpr int kSplitBoxBytes = 8 * kSplitRowBytes;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // every mbarrier wait gives up after 2 s
 
 __device__ FwdFrags g_fwd;
@@ -98,15 +109,21 @@ constexpr int packed_row_bytes() {
   return kIn == kInPack2 ? 64 : kIn == kInPack3 ? 128 : 0;
 }
 
-template <int W, int S, int kIn = kInInt16, bool kWide = false>
+__host__ __device__ constexpr bool split_input(bool inverse, int in, bool wide) {
+  return !inverse && wide && (in == kInInt16 || in == kInSmall);
+}
+
+template <int W, int S, int kIn = kInInt16, bool kWide = false, bool kSplitIn = false>
 struct Cfg {
   static constexpr int kWarps = W;
   static constexpr int kThreads = 32 * W;
   static constexpr int kTile = 8 * W;                 // polynomials per tile
   // a slot: kTile padded rows, then (packed forms) the tile's packed input
   static constexpr int kPackBytes = packed_row_bytes<kIn>();
-  static constexpr int kRowsBytes = kTile * kRowBytes;
-  static constexpr int kSlotBytes = kTile * (kRowBytes + kPackBytes);
+  // bytes from one 8-polynomial unit to the next
+  static constexpr int kUnitBytes = kSplitIn ? kSplitBoxBytes : kWarpBoxBytes;
+  static constexpr int kRowsBytes = W * kUnitBytes;
+  static constexpr int kSlotBytes = kRowsBytes + kTile * kPackBytes;
   static constexpr int kSlots = S;
   // wide kernels: one tile of int32 stage-1 sums after the slots
   static constexpr int kInterBytes = kWide ? kTile * kWideRowBytes : 0;
@@ -170,7 +187,7 @@ __device__ __forceinline__ void block_stage(uint32_t slot, uint8_t* slotp, int b
 // block_stage, two ldmatrix.x4 per block pair (one per block).  ldw[p]: this
 // lane's ldmatrix row offset of pair p's first block (polynomial lane&7 of
 // the n-tile, parity (lane/16) placed by the row swizzle, half (lane/8)&1).
-template <int NT, int P>
+template <int NT, int P, int kUnit = kWarpBoxBytes>
 __device__ __forceinline__ void block_stage_wide(uint32_t inter, uint8_t* slotp, int blk0,
                                                  const uint32_t (&ldw)[P], uint32_t stc_off,
                                                  const uint32_t (&ac)[P][2][2][4]) {
@@ -188,7 +205,7 @@ __device__ __forceinline__ void block_stage_wide(uint32_t inter, uint8_t* slotp,
       ldsm_x4(a1, n[0], n[1], n[2], n[3]);
       ldsm_x4(a1 + 64, n[4], n[5], n[6], n[7]);
     }
-    stage_c_wide(ac[p], r, slotp + nt * 8 * kRowBytes + 32 * (blk0 + 2 * p) + stc_off);
+    stage_c_wide(ac[p], r, slotp + nt * kUnit + 32 * (blk0 + 2 * p) + stc_off);
 #pragma unroll
     for (int j = 0; j < 8; j++) r[j] = n[j];
   }
@@ -331,6 +348,7 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
                                                  int32_t cb_lo, int32_t cb_hi, uint32_t w_even,
                                                  uint32_t w_odd, int lane, uint32_t* bad) {
   constexpr int kOutRow = kWideOut ? kWideRowBytes : kRowBytes;
+  constexpr int kInRow = kWideOut ? kSplitRowBytes : kRowBytes;
   auto out = [&](int p, uint32_t bt0, uint32_t bt1) {
     if constexpr (kWideOut)
       stage_m_small_wide(ab, cb_lo, cb_hi, bt0, bt1, minep + p * kOutRow, w_even, w_odd);
@@ -344,7 +362,7 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
 #pragma unroll
     for (int p = 0; p < kRows; p++) {
       uint32_t nx[4] = {0, 0, 0, 0};
-      if (p + 1 < kRows) ldsm_x4_t(mine + (p + 1) * kRowBytes + ldt_off, nx[0], nx[1], nx[2], nx[3]);
+      if (p + 1 < kRows) ldsm_x4_t(mine + (p + 1) * kInRow + ldt_off, nx[0], nx[1], nx[2], nx[3]);
       const uint32_t bt0 = small_operand(b[0], b[1], bad);
       const uint32_t bt1 = small_operand(b[2], b[3], bad);
       out(p, bt0, bt1);
@@ -384,9 +402,9 @@ __device__ __forceinline__ void poly_stage_small(uint32_t mine, uint8_t* minep, 
   }
 }
 
-// Forward stage 1 of kRows polynomials into the int32 intermediates (wide
-// kernels), the next ldmatrix issued ahead.
-template <int kRows = 8>
+// Forward stage 1 of kRows polynomials (rows kPitch apart) into the int32
+// intermediates (wide kernels), the next ldmatrix issued ahead.
+template <int kRows = 8, int kPitch = kSplitRowBytes>
 __device__ __forceinline__ void poly_stage_fwd_wide(uint32_t rows, uint8_t* irows, uint32_t ldt_off,
                                                     const uint32_t (&am)[2][4], int32_t cm_lo,
                                                     int32_t cm_hi, uint32_t wi_e, uint32_t wi_o) {
@@ -395,7 +413,7 @@ __device__ __forceinline__ void poly_stage_fwd_wide(uint32_t rows, uint8_t* irow
 #pragma unroll
   for (int p = 0; p < kRows; p++) {
     uint32_t n[4] = {0, 0, 0, 0};
-    if (p + 1 < kRows) ldsm_x4_t(rows + (p + 1) * kRowBytes + ldt_off, n[0], n[1], n[2], n[3]);
+    if (p + 1 < kRows) ldsm_x4_t(rows + (p + 1) * kPitch + ldt_off, n[0], n[1], n[2], n[3]);
     stage_m_wide(am, cm_lo, cm_hi, b[0] ^ 0x80008000u, b[1] ^ 0x80008000u, b[2] ^ 0x80008000u,
                  b[3] ^ 0x80008000u, irows + p * kWideRowBytes, wi_e, wi_o);
 #pragma unroll
@@ -406,14 +424,17 @@ __device__ __forceinline__ void poly_stage_fwd_wide(uint32_t rows, uint8_t* irow
 // ------------------------------------------------------------ the kernel ---
 template <bool kInverse, int W, int S, int kIn = kInInt16, bool kAdd = false,
           class Param = OneSeg, bool kWide = false>
-__global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
+__global__ void __launch_bounds__(
+    32 * W, Cfg<W, S, kIn, kWide, split_input(kInverse, kIn, kWide)>::kMinBlocks)
     k_ntt_mma(const __grid_constant__ Param segs) {
   constexpr bool kMulti = std::is_same<Param, SegMaps>::value;
   static_assert(!kInverse || kIn == kInInt16, "input forms are forward only");
   static_assert(kInverse || !kAdd, "the addend is an inverse option");
   static_assert(!kWide || ((kIn == kInInt16 || !kInverse) && !(kMulti && kInverse)),
                 "wide: the inverse with int16 input and one segment");
-  using C = Cfg<W, S, kIn, kWide>;
+  constexpr bool kSplitIn = split_input(kInverse, kIn, kWide);
+  using C = Cfg<W, S, kIn, kWide, kSplitIn>;
+  constexpr int kInRow = kSplitIn ? kSplitRowBytes : kRowBytes;
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -508,7 +529,9 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
   // of block m swapped when bit 2 of m is set, so that the eight rows of each
   // matrix (m = 0..7 or 8..15, 32 bytes apart) fall on eight different bank
   // groups instead of two rows per group.
-  const uint32_t ldt_off = 32u * ((lane & 7) + 8 * ((lane >> 3) & 1)) +
+  // Split input rows have 16 bytes more before every fourth block instead.
+  const uint32_t ldt_m = (uint32_t)((lane & 7) + 8 * ((lane >> 3) & 1));
+  const uint32_t ldt_off = 32u * ldt_m + (kSplitIn ? 16u * (ldt_m >> 2) : 0u) +
                            16u * ((lane >> 4) ^ (kInverse ? (lane >> 2) & 1 : 0));
   // forward stage-1 stores: block i = lane/4 (and +8); the parity halves are
   // swapped in blocks with bit 2 set (bank spread).
@@ -597,9 +620,12 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
         mbar_expect_tx(bar, 8 * C::kPackBytes);
         tma_load_2d(smem0 + slot_i * C::kSlotBytes + C::kRowsBytes + warp * 8 * C::kPackBytes,
                     tm_in, 0, row, bar);
+      } else if (kSplitIn) {
+        mbar_expect_tx(bar, kSplitBoxBytes);
+        tma_load_3d(smem0 + slot_i * C::kSlotBytes + warp * C::kUnitBytes, tm_in, 0, 0, row, bar);
       } else {
         mbar_expect_tx(bar, kWarpBoxBytes);
-        tma_load_2d(smem0 + slot_i * C::kSlotBytes + warp * kWarpBoxBytes, tm_in, 0, row, bar);
+        tma_load_2d(smem0 + slot_i * C::kSlotBytes + warp * C::kUnitBytes, tm_in, 0, row, bar);
       }
     } else {
       mbar_expect_tx(bar, 0);  // arrive only
@@ -611,7 +637,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
     if (unit < u_end) {
       const int sg = seg_of(unit);
       tma_store_2d(map_out(sg), 0, 8 * (unit - seg_first(sg)),
-                   smem0 + slot_i * C::kSlotBytes + warp * kWarpBoxBytes);
+                   smem0 + slot_i * C::kSlotBytes + warp * C::kUnitBytes);
     }
     bulk_commit();
   };
@@ -629,7 +655,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
   auto short_tile = [&](auto nc, uint32_t slot, uint8_t* slotp) {
     constexpr int NU = decltype(nc)::value, R = NU * 8 / W;
     const int row = R * warp;  // this warp's first row in the stages over m
-    const uint32_t rows = slot + row * kRowBytes;
+    [[maybe_unused]] const uint32_t rows = slot + row * kInRow;
     uint8_t* const rowsp = slotp + row * kRowBytes;
     if constexpr (kInverse) {
       if constexpr (kWide)
@@ -645,7 +671,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
         poly_stage<true, false, R>(rows, rowsp, ldt_off, am, cm_lo, cm_hi, cb, 0, 0, w_nat, nullptr,
                                    0, 0, 0);
     } else {
-      uint8_t* const dst = kWide ? interp + row * kWideRowBytes : rowsp;
+      [[maybe_unused]] uint8_t* const dst = kWide ? interp + row * kWideRowBytes : rowsp;
       if constexpr (kIn != kInInt16)
         poly_stage_small<kIn, kWide, R>(rows, dst, ldt_off,
                                         slotp + C::kRowsBytes + row * C::kPackBytes, ab, cb_lo,
@@ -658,7 +684,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
                                     nullptr, 0, 0, 0);
       cta_sync_named();
       if constexpr (kWide)
-        block_stage_wide<NU>(inter, slotp, blk0, ldw, stc_off, ac);
+        block_stage_wide<NU, C::kPairsPerWarp, C::kUnitBytes>(inter, slotp, blk0, ldw, stc_off, ac);
       else
         block_stage<true, false, W, C::kPairsPerWarp, NU>(slot, slotp, blk0, ldc_off, stc_off, ac,
                                                           cc);
@@ -692,7 +718,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
       issue_load(k + C::kSlots - 1, s2);
     }
     // own polynomials of this warp: rows 8w .. 8w+7
-    const uint32_t mine = slot + 8 * warp * kRowBytes;
+    const uint32_t mine = slot + 8 * warp * kInRow;
     uint8_t* minep = slotp + 8 * warp * kRowBytes;
 
     if constexpr (kShortTile) {
@@ -730,7 +756,7 @@ __global__ void __launch_bounds__(32 * W, Cfg<W, S, kIn, kWide>::kMinBlocks)
         if (u_begin + k * W + warp < u_end) bad |= tile_bad;
       }
       cta_sync_named();
-      block_stage_wide<W>(inter, slotp, blk0, ldw, stc_off, ac);
+      block_stage_wide<W, C::kPairsPerWarp, C::kUnitBytes>(inter, slotp, blk0, ldw, stc_off, ac);
       fence_proxy_async_smem();
       cta_sync_named();
       issue_store(k, slot_i);
@@ -967,8 +993,9 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       load_am(g_fwd.s1, fam);
       const uint2 c1 = ldg_keep_u2(&g_fwd.c1[lane][0]);
       constexpr int kR = 2 * NU;  // rows per warp
-      poly_stage_fwd_wide<kR>(slot + kR * warp * kRowBytes, interp + kR * warp * kWideRowBytes,
-                              ldt_off, fam, (int32_t)c1.x, (int32_t)c1.y, wi_e, wi_o);
+      poly_stage_fwd_wide<kR, kRowBytes>(slot + kR * warp * kRowBytes,
+                                         interp + kR * warp * kWideRowBytes, ldt_off, fam,
+                                         (int32_t)c1.x, (int32_t)c1.y, wi_e, wi_o);
     }
     cta_sync_named();
     uint32_t fac[PP][2][2][4];
@@ -984,7 +1011,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
           fac[p][h][s][2] = v.z;
           fac[p][h][s][3] = v.w;
         }
-    block_stage_wide<NU>(inter, slotp, blk0, ldw, stc_off, fac);
+    block_stage_wide<NU, PP>(inter, slotp, blk0, ldw, stc_off, fac);
   };
   // basemul-accumulate in place, one job per warp at a time, its loads of A
   // issued first (k = 4: half of them, which leaves registers and loses no time)
@@ -1098,14 +1125,16 @@ struct Variant {
   // tiles cost less than whole ones (1,000 polynomials on 125 CTAs 1.77 us, on 32
   // CTAs 2.53), else a tile
   int grain;
+  bool split;  // input through encode_split_map
 };
 
 template <bool I, int W, int S, int kIn = kInInt16, bool kAdd = false, class P = OneSeg,
           bool kWide = false>
 constexpr Variant make_variant() {
-  using C = Cfg<W, S, kIn, kWide>;
+  using C = Cfg<W, S, kIn, kWide, split_input(I, kIn, kWide)>;
   return Variant{(const void*)k_ntt_mma<I, W, S, kIn, kAdd, P, kWide>, C::kThreads, C::kSmem,
-                 C::kTile, kAdd || std::is_same<P, SegMaps>::value ? C::kTile : 8};
+                 C::kTile, kAdd || std::is_same<P, SegMaps>::value ? C::kTile : 8,
+                 split_input(I, kIn, kWide)};
 }
 
 // [inverse][variant] (the mma.sync variants; variant 4 is tk_tc5.cu's)
@@ -1152,43 +1181,57 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// The batch as a [npoly][128] uint32 tensor; boxes of 8 polynomials x 132
-// words (the last 4 words are out of bounds: the smem row pad).
-static bool encode_batch_map(CUtensorMap* map, const int16_t* base, int npoly) {
+static bool encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
+                       const cuuint64_t* strides, const cuuint32_t* box) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
   if (!enc) {
     g_last_encode_result = -1;
     return false;
   }
-  const cuuint64_t dims[2] = {128, (cuuint64_t)npoly};
-  const cuuint64_t strides[1] = {512};
-  const cuuint32_t box[2] = {kRowBytes / 4, 8};
-  const cuuint32_t estr[2] = {1, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r =
-      enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)base, dims, strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+      enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, (cuuint32_t)rank, (void*)base, dims, strides, box,
+          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   g_last_encode_result = (int)r;
   return r == CUDA_SUCCESS;
 }
 
+// The batch as a [npoly][128] uint32 tensor; boxes of 8 polynomials x 132
+// words (the last 4 words are out of bounds: the smem row pad).
+static bool encode_batch_map(CUtensorMap* map, const int16_t* base, int npoly) {
+  const cuuint64_t dims[2] = {128, (cuuint64_t)npoly};
+  const cuuint64_t strides[1] = {512};
+  const cuuint32_t box[2] = {kRowBytes / 4, 8};
+  return encode_map(map, base, 2, dims, strides, box);
+}
+
+// The batch as a [npoly][4][32] uint32 tensor; boxes of 8 polynomials x 4 quarters
+// x 36 words (the last 4 out of bounds: the pad of kSplitRowBytes).
+static bool encode_split_map(CUtensorMap* map, const int16_t* base, int npoly) {
+  const cuuint64_t dims[3] = {32, 4, (cuuint64_t)npoly};
+  const cuuint64_t strides[2] = {128, 512};
+  const cuuint32_t box[3] = {36, 4, 8};
+  return encode_map(map, base, 3, dims, strides, box);
+}
+
 // A packed batch as a [npoly][row_bytes / 4] uint32 tensor, boxes of 8 rows.
 static bool encode_packed_map(CUtensorMap* map, const void* base, int npoly, int row_bytes) {
-  PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
-  if (!enc) {
-    g_last_encode_result = -1;
-    return false;
-  }
   const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 4), (cuuint64_t)npoly};
   const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
   const cuuint32_t box[2] = {(cuuint32_t)(row_bytes / 4), 8};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r =
-      enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)base, dims, strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  g_last_encode_result = (int)r;
-  return r == CUDA_SUCCESS;
+  return encode_map(map, base, 2, dims, strides, box);
+}
+
+// The input and output maps of one batch on a kernel's layouts.
+static bool encode_io(bool split, CUtensorMap* in, CUtensorMap* out, const int16_t* src,
+                      int16_t* dst, int npoly) {
+  if (!(split ? encode_split_map(in, src, npoly) : encode_batch_map(in, src, npoly))) return false;
+  if (!split && src == dst) {
+    *out = *in;
+    return true;
+  }
+  return encode_batch_map(out, dst, npoly);
 }
 
 int last_encode_result() { return g_last_encode_result; }
@@ -1324,13 +1367,12 @@ cudaError_t launch_fwd_form(int form, const void* src, int16_t* dst, long long n
       continue;
     }
     OneSeg m = {};
-    const bool ok_in = form == kInSmall ? encode_batch_map(&m.in, (const int16_t*)in, n)
-                                        : encode_packed_map(&m.in, in, n, row_bytes);
-    if (!ok_in) return cudaErrorInvalidResourceHandle;
-    if ((const void*)in == (const void*)(dst + done * 256))
-      m.out = m.in;
-    else if (!encode_batch_map(&m.out, dst + done * 256, n))
-      return cudaErrorInvalidResourceHandle;
+    const bool ok =
+        form == kInSmall
+            ? encode_io(V.split, &m.in, &m.out, (const int16_t*)in, dst + done * 256, n)
+            : encode_packed_map(&m.in, in, n, row_bytes) &&
+                  encode_batch_map(&m.out, dst + done * 256, n);
+    if (!ok) return cudaErrorInvalidResourceHandle;
     m.npoly = n;
     const cudaError_t e = launch_variant(V, cap, m, n, stream);
     if (e != cudaSuccess) return e;
@@ -1375,10 +1417,7 @@ cudaError_t launch_mma_segs(bool inverse, int variant, const Seg* segs, int nseg
                             (add_form ? info.add_ctas_per_sm[variant]
                                       : info.mma_ctas_per_sm[inverse ? 1 : 0][variant]);
       OneSeg m = {};
-      if (!encode_batch_map(&m.in, pc[0].src, pc[0].n)) return cudaErrorInvalidResourceHandle;
-      if (pc[0].src == pc[0].dst)
-        m.out = m.in;
-      else if (!encode_batch_map(&m.out, pc[0].dst, pc[0].n))
+      if (!encode_io(V.split, &m.in, &m.out, pc[0].src, pc[0].dst, pc[0].n))
         return cudaErrorInvalidResourceHandle;
       m.addend = (const uint32_t*)pc[0].addend;
       m.npoly = pc[0].n;
@@ -1391,10 +1430,7 @@ cudaError_t launch_mma_segs(bool inverse, int variant, const Seg* segs, int nseg
     SegMaps m = {};
     int units = 0;
     for (int k = 0; k < np; k++) {
-      if (!encode_batch_map(&m.in[k], pc[k].src, pc[k].n)) return cudaErrorInvalidResourceHandle;
-      if (pc[k].src == pc[k].dst)
-        m.out[k] = m.in[k];
-      else if (!encode_batch_map(&m.out[k], pc[k].dst, pc[k].n))
+      if (!encode_io(V.split, &m.in[k], &m.out[k], pc[k].src, pc[k].dst, pc[k].n))
         return cudaErrorInvalidResourceHandle;
       m.addend[k] = (const uint32_t*)pc[k].addend;
       m.npoly[k] = pc[k].n;
@@ -1437,10 +1473,7 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
     // rows are 32-bit TMA coordinates and tile numbers 32-bit integers
     if (B.njobs * (size_t)B.k > (size_t)kMaxLaunchPolys) return cudaErrorInvalidValue;
     const int nvec = (int)(B.njobs * B.k);
-    if (!encode_batch_map(&m.s_map[b], B.s, nvec)) return cudaErrorInvalidResourceHandle;
-    if (B.out == B.s)
-      m.out_map[b] = m.s_map[b];
-    else if (!encode_batch_map(&m.out_map[b], B.out, nvec))
+    if (!encode_io(false, &m.s_map[b], &m.out_map[b], B.s, B.out, nvec))
       return cudaErrorInvalidResourceHandle;
     m.A[b] = B.A;
     m.e[b] = (const uint32_t*)B.e;

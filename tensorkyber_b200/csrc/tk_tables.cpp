@@ -314,7 +314,7 @@ void build_pack_tables(int bits, uint8_t* out) {
   for (int h = 0; h < 2; h++)
     for (int m = 0; m < 64; m++) {
       // row 2m over j = 2i + h: c0 in [-unit/2, unit/2), c1 = (c - c0) / unit
-      int c[64], c0[64], sum = 0;
+      int c[64] = {}, c0[64] = {}, sum = 0;
       auto split = [&](int i) { c0[i] = ((c[i] + unit / 2) & (unit - 1)) - unit / 2; };
       for (int i = 0; i < 64; i++) {
         c[i] = F[2 * m][2 * i + h];
