@@ -161,9 +161,9 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
   }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = (int)gridDim.x;
-  const int t_begin = (int)((long long)blockIdx.x * P.ntiles / G);
-  const int t_end = (int)((long long)(blockIdx.x + 1) * P.ntiles / G);
-  const int nmine = t_end - t_begin;
+  // tiles round robin: the launch moves through the batch as one front
+  const int nmine = (P.ntiles - 1 - (int)blockIdx.x) / G + 1;
+  auto tile_row = [&](int k) { return kPkTile * (k * G + (int)blockIdx.x); };
 
   const uint32_t bars = base + L::kOffBars;
   constexpr int S = L::kInSlots;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
         if (k >= S && !(ok = mbar_wait_bounded(in_empty(s), (uint32_t)(k / S - 1) & 1u, kPkWaitNs)))
           break;
         mbar_expect_tx(in_full(s), L::kInBytes);
-        tma_load_2d(base + L::kOffIn + s * L::kInBytes, &P.in, 0, kPkTile * (t_begin + k),
+        tma_load_2d(base + L::kOffIn + s * L::kInBytes, &P.in, 0, tile_row(k),
                     in_full(s));
       }
       // every load has landed before the CTA's memory goes
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
         const int b = k % NO;
         for (int g = 0; g < 4; g++) {
           if (!(ok = mbar_wait_bounded(out_ready(b, g), (uint32_t)(k / NO) & 1u, kPkWaitNs))) break;
-          tma_store_2d(&P.out, 64 * g, kPkTile * (t_begin + k),
+          tma_store_2d(&P.out, 64 * g, tile_row(k),
                        base + L::kOffOut + b * kPkOutSlot + g * kPkOutBox);
           bulk_commit();
         }

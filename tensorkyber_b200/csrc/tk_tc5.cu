@@ -170,9 +170,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
   }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = (int)gridDim.x;
-  const int t_begin = (int)((long long)blockIdx.x * P.ntiles / G);
-  const int t_end = (int)((long long)(blockIdx.x + 1) * P.ntiles / G);
-  const int nmine = t_end - t_begin;
+  // tiles round robin, the whole launch one front through the batch: upwards in
+  // the forward, downwards in the inverse, which then starts on what a forward on
+  // the same memory wrote last (as the mma.sync kernels)
+  const int nmine = (P.ntiles - 1 - (int)blockIdx.x) / G + 1;
+  auto tile_row = [&](int k) {
+    const int t = k * G + (int)blockIdx.x;
+    return kTcTile * (kInverse ? P.ntiles - 1 - t : t);
+  };
 
   const uint32_t tables = base + kOffTables;
   const uint32_t bars = base + L::kOffBars;
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
       auto load = [&](int k) {
         const int s = k % kTcSlots;
         mbar_expect_tx(in_full(s), kTcSlotBytes);
-        const int row = kTcTile * (t_begin + k);
+        const int row = tile_row(k);
         for (int q = 0; q < 4; q++)
           tma_load_2d(slot_addr(s) + q * kTcQuarterBytes, &P.in, 64 * q, row, in_full(s));
         last_load[s] = k;
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
           ok = false;
           break;
         }
-        const int row = kTcTile * (t_begin + k);
+        const int row = tile_row(k);
         for (int q = 0; q < 4; q++)
           tma_store_2d(&P.out, 64 * q, row, slot_addr(s) + q * kTcQuarterBytes);
         bulk_commit();
