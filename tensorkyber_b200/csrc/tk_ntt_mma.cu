@@ -821,7 +821,8 @@ __global__ void __launch_bounds__(
 //     out_i = invntt( sum_j basemul(A_ij, ntt(s_j)) ) + e_i,
 // with all three steps on one CTA's shared memory.  A tile is kJobs(k)
 // consecutive jobs of one batch, i.e. kRows(k) = kJobs * k consecutive vector
-// rows of its s / e / out (32 for k = 2, 4; 24 for k = 3): 8-row TMA boxes in,
+// rows of its s / e / out (32 for k = 2, 4; 24 for k = 3; small calls run smaller
+// tiles, kUnits = 2 or 1): 8-row TMA boxes in,
 // the forward NTT in place (the batch kernels' stages: by polynomial, CTA
 // barrier, by block over the tile's n-tiles), the basemul-accumulate by job in
 // place over ntt(s) (warp w: jobs w, w+4, ...; a job's rows are read whole before
@@ -876,9 +877,22 @@ __device__ InvFrags g_tile_inv;
 constexpr int kTileSlotBytes = 32 * kRowBytes;      // one 32-row slot
 constexpr int kTileWideBytes = 32 * kWideRowBytes;  // the forward's int32 sums
 constexpr int kTileSmem = kTileSlotBytes + kTileWideBytes + 16;  // and an mbarrier
-__host__ __device__ constexpr int tile_units(int k) { return k == 3 ? 3 : 4; }
-__host__ __device__ constexpr int tile_jobs(int k) { return 8 * tile_units(k) / k; }
+// Tiles of a launch of kind `units` (4, 2 or 1): 8-row shared-memory units, rows of
+// the batch and jobs per tile.  k = 3: 24 rows, the smallest whole number of both
+// jobs and units, or, with units = 1, two jobs in six rows of one unit (six-row
+// TMA boxes).
+__host__ __device__ constexpr int tile_units(int k, int units) {
+  return k == 3 && units > 1 ? 3 : units;
+}
+__host__ __device__ constexpr int tile_box_rows(int k, int units) {
+  return k == 3 && units == 1 ? 6 : 8;
+}
+__host__ __device__ constexpr int tile_rows(int k, int units) {
+  return tile_units(k, units) * tile_box_rows(k, units);
+}
+__host__ __device__ constexpr int tile_jobs(int k, int units) { return tile_rows(k, units) / k; }
 
+template <int kUnits>
 __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__ MvTiles P) {
   constexpr int W = 4, PP = 2;  // PP: block pairs per warp
   extern __shared__ __align__(128) uint8_t smem[];
@@ -977,9 +991,9 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   auto issue_load = [&](int k) {
     if (lane != 0) return;
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), kb = P.k[b];
-    const int row = (t - P.first_tile[b]) * 8 * tile_units(kb) + 8 * warp;
-    if (warp < tile_units(kb) && row < P.njobs[b] * kb) {  // boxes past the batch: none
-      mbar_expect_tx(bar0, kWarpBoxBytes);
+    const int row = (t - P.first_tile[b]) * tile_rows(kb, kUnits) + 8 * warp;
+    if (warp < tile_units(kb, kUnits) && row < P.njobs[b] * kb) {  // boxes past the batch: none
+      mbar_expect_tx(bar0, tile_box_rows(kb, kUnits) * kRowBytes);
       tma_load_2d(slot + warp * kWarpBoxBytes, &P.s_map[b], 0, row, bar0);
     } else {
       mbar_expect_tx(bar0, 0);  // arrive only
@@ -992,8 +1006,8 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   auto prefetch = [&](int k) {
     if (tid != 0) return;
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), kb = P.k[b];
-    const int j0 = (t - P.first_tile[b]) * tile_jobs(kb);
-    const int nj = min(tile_jobs(kb), P.njobs[b] - j0);
+    const int j0 = (t - P.first_tile[b]) * tile_jobs(kb, kUnits);
+    const int nj = min(tile_jobs(kb, kUnits), P.njobs[b] - j0);
     bulk_prefetch_l2(P.A[b] + (size_t)j0 * kb * kb * 256, (uint32_t)nj * kb * kb * 512u);
     if (P.e[b]) bulk_prefetch_l2(P.e[b] + (size_t)j0 * kb * 128, (uint32_t)nj * kb * 512u);
   };
@@ -1032,7 +1046,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   // issued first (k = 4: half of them, which leaves registers and loses no time)
   auto basemul_phase = [&](auto kc, int b, int tl) {
     constexpr int K = decltype(kc)::value;
-    constexpr int kJobs = tile_jobs(K);
+    constexpr int kJobs = tile_jobs(K, kUnits);
     const int njobs = P.njobs[b];
     for (int jl = warp; jl < kJobs; jl += W) {
       const int job = tl * kJobs + jl;
@@ -1093,8 +1107,8 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       tma_store_2d(&P.out_map[b], 0, row0 + 8 * warp, slot + warp * kWarpBoxBytes);
     if (lane == 0) bulk_commit();  // every lane-0 keeps one (possibly empty) group per tile
   };
-  using U3 = std::integral_constant<int, 3>;
-  using U4 = std::integral_constant<int, 4>;
+  using U3 = std::integral_constant<int, kUnits == 1 ? 1 : 3>;
+  using UN = std::integral_constant<int, kUnits>;
 
   issue_load(0);
   for (int k = 0; k < nmine; k++) {
@@ -1106,11 +1120,11 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     prefetch(k);
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), tl = t - P.first_tile[b];
     const int kb = P.k[b];  // CTA-uniform
-    const int row0 = tl * 8 * tile_units(kb), nvec = P.njobs[b] * kb;
-    if (tile_units(kb) == 3)  // the phase code for the tile's unit count
+    const int row0 = tl * tile_rows(kb, kUnits), nvec = P.njobs[b] * kb;
+    if (kUnits > 1 && tile_units(kb, kUnits) == 3)  // the phase code for the tile's unit count
       fwd_phase(U3{});
     else
-      fwd_phase(U4{});
+      fwd_phase(UN{});
     cta_sync_named();
     switch (kb) {
       case 2: basemul_phase(std::integral_constant<int, 2>{}, b, tl); break;
@@ -1118,10 +1132,10 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       default: basemul_phase(std::integral_constant<int, 4>{}, b, tl); break;
     }
     cta_sync_named();
-    if (tile_units(kb) == 3)  // the phase code for the tile's unit count
+    if (kUnits > 1 && tile_units(kb, kUnits) == 3)  // the phase code for the tile's unit count
       inv_phase(U3{}, b, row0, nvec);
     else
-      inv_phase(U4{}, b, row0, nvec);
+      inv_phase(UN{}, b, row0, nvec);
     if (k + 1 < nmine) {
       if (lane == 0) bulk_wait_read<0>();  // this lane's own box
       issue_load(k + 1);
@@ -1212,12 +1226,12 @@ static bool encode_map(CUtensorMap* map, const void* base, int rank, const cuuin
   return r == CUDA_SUCCESS;
 }
 
-// The batch as a [npoly][128] uint32 tensor; boxes of 8 polynomials x 132
+// The batch as a [npoly][128] uint32 tensor; boxes of 8 (box_rows) polynomials x 132
 // words (the last 4 words are out of bounds: the smem row pad).
-static bool encode_batch_map(CUtensorMap* map, const int16_t* base, int npoly) {
+static bool encode_batch_map(CUtensorMap* map, const int16_t* base, int npoly, int box_rows = 8) {
   const cuuint64_t dims[2] = {128, (cuuint64_t)npoly};
   const cuuint64_t strides[1] = {512};
-  const cuuint32_t box[2] = {kRowBytes / 4, 8};
+  const cuuint32_t box[2] = {kRowBytes / 4, (cuuint32_t)box_rows};
   return encode_map(map, base, 2, dims, strides, box);
 }
 
@@ -1240,13 +1254,14 @@ static bool encode_packed_map(CUtensorMap* map, const void* base, int npoly, int
 
 // The input and output maps of one batch on a kernel's layouts.
 static bool encode_io(bool split, CUtensorMap* in, CUtensorMap* out, const int16_t* src,
-                      int16_t* dst, int npoly) {
-  if (!(split ? encode_split_map(in, src, npoly) : encode_batch_map(in, src, npoly))) return false;
+                      int16_t* dst, int npoly, int box_rows = 8) {
+  if (!(split ? encode_split_map(in, src, npoly) : encode_batch_map(in, src, npoly, box_rows)))
+    return false;
   if (!split && src == dst) {
     *out = *in;
     return true;
   }
-  return encode_batch_map(out, dst, npoly);
+  return encode_batch_map(out, dst, npoly, box_rows);
 }
 
 int last_encode_result() { return g_last_encode_result; }
@@ -1276,6 +1291,12 @@ static bool upload_tables_current_device() {
   if (cudaMemcpyToSymbol(g_tile_z, z, sizeof(z)) != cudaSuccess) return false;
   const unsigned zero = 0;
   return cudaMemcpyToSymbol(g_status, &zero, sizeof(zero)) == cudaSuccess;
+}
+
+static const void* tile_fn(int units) {
+  return units == 4   ? (const void*)k_matvec_tiles<4>
+         : units == 2 ? (const void*)k_matvec_tiles<2>
+                      : (const void*)k_matvec_tiles<1>;
 }
 
 bool mma_init_device(DeviceInfo* info) {
@@ -1318,14 +1339,18 @@ bool mma_init_device(DeviceInfo* info) {
     info->multi_ctas_per_sm[m] = per_sm > 0 ? per_sm : 1;
   }
   {
-    const void* fn = (const void*)k_matvec_tiles;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem) !=
-        cudaSuccess)
-      return false;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, kTileSmem) != cudaSuccess)
-      return false;
-    info->tile_ctas_per_sm = per_sm > 0 ? per_sm : 1;
+    info->tile_ctas_per_sm = 1 << 20;
+    for (int units = 4; units >= 1; units >>= 1) {
+      const void* fn = tile_fn(units);
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem) !=
+          cudaSuccess)
+        return false;
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, kTileSmem) != cudaSuccess)
+        return false;
+      per_sm = per_sm > 0 ? per_sm : 1;
+      if (per_sm < info->tile_ctas_per_sm) info->tile_ctas_per_sm = per_sm;
+    }
   }
   for (int f = 0; f < kNumInputForms; f++) {
     const Variant& V = kFormVariants[f];
@@ -1482,25 +1507,50 @@ cudaError_t launch_mma(bool inverse, int variant, const int16_t* src, int16_t* d
 cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceInfo& info,
                                cudaStream_t stream) {
   if (nb > kMaxSegs) return cudaErrorInvalidValue;
+  const long long cap = (long long)info.num_sms * info.tile_ctas_per_sm;
+  // Tile kind: the smallest tiles that make one round of resident CTAs (592), since
+  // a tile's latency is what a small call costs.  Half tiles with k = 3 batches
+  // (whose tiles they do not shorten) only within two CTAs per SM, or where whole
+  // tiles go beyond that themselves.  us, 1 / 2 / 4 units: 24 jobs of k = 3 3.0 / 5.4 /
+  // 5.4; 37 of k = 4 3.4 / 4.5 / 6.4; 341 of each k 5.3 / 6.1 / 6.7 (428 / 172 / 108
+  // tiles); 1,500 of k = 4 8.6 / 7.9 / 8.9; 500 of each 6.7 / 6.4 / 8.3; 900 of each
+  // 9.2 / 9.5 / 8.7 (451 half, 283 whole tiles); 1,100 of each 12.1 / 9.7 / 12.5;
+  // 8,000 of k = 2 15.9 / 14.4 / 13.1.
+  auto tiles_of = [&](int units) {
+    size_t tiles = 0;
+    for (int b = 0; b < nb; b++) {
+      const size_t tj = (size_t)tile_jobs(batches[b].k, units);
+      tiles += (batches[b].njobs + tj - 1) / tj;
+    }
+    return tiles;
+  };
+  bool any3 = false;
+  for (int b = 0; b < nb; b++) any3 |= batches[b].k == 3;
+  const size_t two = 2 * (size_t)info.num_sms;
+  const int units = tiles_of(1) <= (size_t)cap ? 1
+                    : tiles_of(2) <= (size_t)cap &&
+                            (!any3 || tiles_of(2) <= two || tiles_of(4) > two)
+                        ? 2
+                        : 4;
   MvTiles m = {};
   for (int b = 0; b < nb; b++) {
     const MatvecPart& B = batches[b];
     // rows are 32-bit TMA coordinates and tile numbers 32-bit integers
     if (B.njobs * (size_t)B.k > (size_t)kMaxLaunchPolys) return cudaErrorInvalidValue;
     const int nvec = (int)(B.njobs * B.k);
-    if (!encode_io(false, &m.s_map[b], &m.out_map[b], B.s, B.out, nvec))
+    if (!encode_io(false, &m.s_map[b], &m.out_map[b], B.s, B.out, nvec,
+                   tile_box_rows(B.k, units)))
       return cudaErrorInvalidResourceHandle;
     m.A[b] = B.A;
     m.e[b] = (const uint32_t*)B.e;
     m.njobs[b] = (int)B.njobs;
     m.k[b] = B.k;
-    const int tj = tile_jobs(B.k);
+    const int tj = tile_jobs(B.k, units);
     m.first_tile[b + 1] = m.first_tile[b] + (int)((B.njobs + tj - 1) / tj);
   }
   m.nb = nb;
   long long ctas = m.first_tile[nb];
   if (ctas <= 0) return cudaSuccess;
-  const long long cap = (long long)info.num_sms * info.tile_ctas_per_sm;
   if (ctas > cap) ctas = cap;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
@@ -1513,7 +1563,7 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   void* args[1] = {(void*)&m};
-  return cudaLaunchKernelExC(&cfg, (const void*)k_matvec_tiles, args);
+  return cudaLaunchKernelExC(&cfg, tile_fn(units), args);
 }
 
 // Self-test of the give-up path: one CTA waits, through the same bounded
