@@ -120,11 +120,14 @@ typedef struct tk_matvec_batch {
   int16_t *out;
 } tk_matvec_batch;
 int tk_matvec(const tk_matvec_batch *batches, int nbatches, tk_stream_t stream);
-/* tk_matvec on HOST buffers, synchronous: copies A, s, e in (one copy when
- * they are contiguous, A then s then e), runs the same kernels, copies out
- * back (the plain per-request launch).  Uses a device
- * staging buffer per device that grows to the largest call (at most 8 GiB);
- * calls on one device are serialised.  out may alias s. */
+/* tk_matvec on HOST buffers, synchronous (the plain per-request launch).
+ * Page-locked, device-mapped buffers are used in place: the kernel writes out
+ * straight to them, and reads A, s and e there when all of them are page-locked
+ * too and no out overlaps any of them (its own s exactly is fine).  What is not
+ * goes through a device staging buffer per device that grows to the largest
+ * call (at most 8 GiB, also for calls that need none of it), inputs in one copy
+ * when they are contiguous, A then s then e.  Calls on one device are
+ * serialised.  out may alias s. */
 int tk_matvec_host(const tk_matvec_batch *batches, int nbatches);
 /* tk_matvec_host for callers that must not allocate (no counterpart in the
  * reference): services that reserve their device memory once at start-up and

@@ -172,6 +172,9 @@ int api_device_info(int device, DeviceInfo** info);
 // allocation (a copy that runs from one page-locked allocation into the next
 // is not valid).  Needs the device's context current on the calling thread.
 bool host_span_one_copy(const void* p, size_t bytes);
+// Device address of [p, p + bytes) when all of it lies in one page-locked,
+// device-mapped host allocation; nullptr otherwise.
+const void* mapped_host_range(const void* p, size_t bytes);
 
 // Forward transform of npoly polynomials given in input form `form` (1..3):
 // src holds int16 rows (form 1; src == dst for in place) or packed rows of

@@ -199,27 +199,6 @@ cudaError_t set_u32(unsigned int* dst, unsigned int v, cudaStream_t st) {
              : cudaErrorLaunchFailure;
 }
 
-// Device address of [p, p + bytes) when all of it lies in one page-locked,
-// device-mapped host allocation; nullptr otherwise (the request is staged).
-const void* mapped_host_range(const void* p, size_t bytes) {
-  static const auto get_attr = driver_fn<PFN_cuPointerGetAttribute_v4000>("cuPointerGetAttribute");
-  if (!p || !get_attr) return nullptr;
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-  CUdeviceptr start = 0;
-  size_t size = 0;
-  const CUdeviceptr dp = (CUdeviceptr)a.devicePointer;
-  if (get_attr(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, dp) != CUDA_SUCCESS ||
-      get_attr(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, dp) != CUDA_SUCCESS)
-    return nullptr;
-  if (dp < start || dp + bytes > start + size) return nullptr;
-  return a.devicePointer;
-}
-
 // The host range [lo, hi) of the page-locked allocation holding p, or false
 // (pageable memory, or no range query).
 bool locked_allocation(const void* p, uintptr_t* lo, uintptr_t* hi) {
@@ -615,12 +594,12 @@ int tk_server_submit(tk_server* S, int k, size_t njobs, const int16_t* A, const 
     cudaSetDevice(S->device);
     // outputs go straight to out whenever it is device-mapped page-locked
     // memory: posted writes over PCIe, no copy back
-    r->dout = (int16_t*)mapped_host_range(out, vb);
+    r->dout = (int16_t*)tk::mapped_host_range(out, vb);
     r->out_direct = r->dout != nullptr;
     if (S->zero_copy) {
-      const void* dA = mapped_host_range(A, ab);
-      const void* ds = dA ? mapped_host_range(s, vb) : nullptr;
-      const void* de = ds && e ? mapped_host_range(e, vb) : nullptr;
+      const void* dA = tk::mapped_host_range(A, ab);
+      const void* ds = dA ? tk::mapped_host_range(s, vb) : nullptr;
+      const void* de = ds && e ? tk::mapped_host_range(e, vb) : nullptr;
       if (ds && (de || !e)) {
         r->in_direct = true;
         r->dA = (const int16_t*)dA;
