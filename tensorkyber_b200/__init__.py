@@ -358,7 +358,8 @@ def matvec_host_noalloc(batches, stream=0):
 
 
 def matvec_host(batches):
-    """tk_matvec on numpy int16 host arrays (synchronous; same shapes as matvec)."""
+    """tk_matvec on numpy int16 host arrays (synchronous; same shapes as matvec;
+    page-locked arrays are used in place)."""
     items = []
     for k, A, s, e, out in batches:
         n = _host_arr(s) // k

@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(
 // constants are re-read from L1 at each stage, so that between stages their
 // registers hold the basemul's loads in flight.  Every mbarrier wait is
 // bounded (2 s; sets status bit 4 and stops the CTA).
-// Bound by instruction issue and load latency (16 warps per SM at about half
+// Bound by instruction issue and load latency (16 warps per SM at 39 % of
 // the issue slots), not DRAM, so instructions come out wherever an
 // intermediate's form is this kernel's own: ntt(s) reduced lazily, A words
 // multiplied packed (dp2a), the accumulators written parity-split and unbiased
@@ -853,9 +853,11 @@ __global__ void __launch_bounds__(
 // warps, six rows each, instead of eight on three: k = 3 alone 70.2 -> 66.4 us,
 // the mix 129.6 -> 126.3.  The forward on int32 sums as the batch kernel's variant
 // 3 (20 instructions per polynomial fewer), in the room of the second slot: 125.5
-// -> 121.8 us, 16,383 jobs 36.8 -> 36.0 (in a long loop 39.9 -> 37.5), 37 jobs of k
-// = 4 6.7 -> 6.4; with both slots kept, three CTAs per SM, 129 us.  Five or six CTAs per SM at 96 or 80 registers:
-// 133.2 / 132.6 us.
+// -> 121.8 us, 16,383 jobs 36.8 -> 36.0 (in a long loop 39.9 -> 37.5); with both
+// slots kept, three CTAs per SM, 129 us.  Five or six CTAs per SM at 96 or 80
+// registers: 133.2 / 132.6 us.  Smaller tiles in calls that leave CTAs idle: 24
+// jobs of k = 3 5.3 -> 3.0 us, 2,000 of k = 2 6.6 -> 4.9 (the rule stands at
+// launch_matvec_tile).
 struct MvTiles {
   CUtensorMap s_map[kMaxSegs];    // s rows [njobs * k][128 words], 8 x 132-word boxes
   CUtensorMap out_map[kMaxSegs];  // out rows, the same shape (may equal s_map: in place)
