@@ -491,7 +491,8 @@ static int validate_matvec(const tk_matvec_batch* batches, int nbatches, bool ho
 
 // Launches a validated batch list of device buffers.
 static int launch_matvec_batches(const tk_matvec_batch* batches, int nbatches,
-                                 const DeviceInfo* info, cudaStream_t stream) {
+                                 const DeviceInfo* info, cudaStream_t stream,
+                                 bool host_inputs = false) {
   const int mode = g_matvec_mode.load(std::memory_order_relaxed);
   if (mode == TK_MATVEC_TILED) {  // one tile-kernel launch per kMaxSegs batches
     tk::MatvecPart parts[tk::kMaxSegs];
@@ -502,7 +503,7 @@ static int launch_matvec_batches(const tk_matvec_batch* batches, int nbatches,
         parts[np++] = tk::MatvecPart{B.k, B.njobs, B.A, B.s, B.e, B.out};
       }
       if (np == tk::kMaxSegs || (b == nbatches && np > 0)) {
-        cudaError_t e = tk::launch_matvec_tile(parts, np, *info, stream);
+        cudaError_t e = tk::launch_matvec_tile(parts, np, *info, stream, host_inputs);
         if (e != cudaSuccess) {
           set_launch_err(e);
           return TK_ERR_CUDA;
@@ -698,7 +699,7 @@ int tk_matvec_host(const tk_matvec_batch* batches, int nbatches) {
     D.out = direct ? direct_out : dout;
   }
   if (e == cudaSuccess) {
-    rc = launch_matvec_batches(dev_batches.data(), nbatches, info, st);
+    rc = launch_matvec_batches(dev_batches.data(), nbatches, info, st, direct == 2);
     if (rc) {
       cudaStreamSynchronize(st);
       return rc;

@@ -123,9 +123,10 @@ cudaError_t launch_matvec(const MatvecPart* batches, int nb, const DeviceInfo& i
                           long long chunk_vec_polys);
 // The tiled single-kernel form: one k_matvec_tiles launch for up to kMaxSegs
 // batches (forward NTT, basemul-accumulate and inverse NTT + e of a tile of
-// jobs in one CTA's shared memory).
+// jobs in one CTA's shared memory).  host_inputs: A, s and e are mapped host
+// memory.
 cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceInfo& info,
-                               cudaStream_t stream);
+                               cudaStream_t stream, bool host_inputs = false);
 
 // ---- serving loop (device side in tk_matvec.cu, host side in tk_serve.cpp) ----
 // One job descriptor of the job ring (64 bytes; the ring lives in mapped

@@ -289,8 +289,9 @@ __device__ __forceinline__ void poly_stage_inv_wide(uint32_t irow0, uint8_t* min
 // Stage over m for this warp's 8 polynomials, the next ldmatrix issued ahead.
 // Inverse with kAdd only: polynomial p of this warp (global index poly0 + p)
 // gets addend[poly0 + p] added to its output; the addend words for
-// polynomial p+1 are fetched while p is computed.
-template <bool kInverse, bool kAdd = false, int kRows = 8>
+// polynomial p+1 are fetched while p is computed.  kAddShared: addend is in
+// shared memory.
+template <bool kInverse, bool kAdd = false, int kRows = 8, bool kAddShared = false>
 __device__ __forceinline__ void poly_stage(uint32_t mine, uint8_t* minep, uint32_t ldt_off,
                                            const uint32_t (&am)[2][4], int32_t cm_lo,
                                            int32_t cm_hi, const int32_t (&cb)[2][4],
@@ -301,10 +302,10 @@ __device__ __forceinline__ void poly_stage(uint32_t mine, uint8_t* minep, uint32
     const int poly = poly0 + p;
     if (kInverse && kAdd && addend != nullptr && poly < npoly) {
       const uint32_t* w = addend + (size_t)poly * 128 + add_off;
-      e[0] = __ldg(w);
-      e[1] = __ldg(w + 4);
-      e[2] = __ldg(w + 64);
-      e[3] = __ldg(w + 68);
+      e[0] = kAddShared ? w[0] : __ldg(w);
+      e[1] = kAddShared ? w[4] : __ldg(w + 4);
+      e[2] = kAddShared ? w[64] : __ldg(w + 64);
+      e[3] = kAddShared ? w[68] : __ldg(w + 68);
     } else {
       e[0] = e[1] = e[2] = e[3] = 0;
     }
@@ -876,9 +877,17 @@ __device__ int32_t g_tile_z[128];  // basemul pair roots z_t (build_pair_roots)
 __device__ TileFrags g_tile_sa;
 __device__ InvFrags g_tile_inv;
 
-constexpr int kTileSlotBytes = 32 * kRowBytes;      // one 32-row slot
-constexpr int kTileWideBytes = 32 * kWideRowBytes;  // the forward's int32 sums
-constexpr int kTileSmem = kTileSlotBytes + kTileWideBytes + 16;  // and an mbarrier
+// Shared memory of a CTA: the slot, the forward's int32 sums, in the staged form A
+// (16 KB) and e of the tile, and two mbarriers.
+struct TileSmem {
+  int wide, A, e, bars, bytes;
+};
+__host__ __device__ constexpr TileSmem tile_smem(bool staged) {
+  const int rows = staged ? 8 : 32;
+  const int wide = rows * kRowBytes, A = wide + rows * kWideRowBytes;
+  const int e = A + (staged ? 8 * 4 * 512 : 0), bars = e + (staged ? 8 * 512 : 0);
+  return TileSmem{wide, A, e, bars, bars + 16};
+}
 // Tiles of a launch of kind `units` (4, 2 or 1): 8-row shared-memory units, rows of
 // the batch and jobs per tile.  k = 3: 24 rows, the smallest whole number of both
 // jobs and units, or, with units = 1, two jobs in six rows of one unit (six-row
@@ -894,7 +903,11 @@ __host__ __device__ constexpr int tile_rows(int k, int units) {
 }
 __host__ __device__ constexpr int tile_jobs(int k, int units) { return tile_rows(k, units) / k; }
 
-template <int kUnits>
+// kStaged (one-unit tiles, one per CTA, on host memory): A and e of the tile come into
+// shared memory beside s, so that a call waits for the link once, not for s, A and e
+// in turn.  Host to host, us: 1 job of k = 3 18.2 -> 15.7, 5 of k = 4 21.0 -> 17.7, 20 of
+// k = 3 21.4 -> 19.2, 36 of k = 4 27.7 -> 27.1.  On device memory the extra hop costs 0.1 us of 2.8.
+template <int kUnits, bool kStaged>
 __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__ MvTiles P) {
   constexpr int W = 4, PP = 2;  // PP: block pairs per warp
   extern __shared__ __align__(128) uint8_t smem[];
@@ -908,9 +921,11 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   const int nmine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / G + 1 : 0;
   const uint32_t slot = smem_u32(smem);
   uint8_t* const slotp = smem;
-  const uint32_t inter = slot + kTileSlotBytes;
-  uint8_t* const interp = smem + kTileSlotBytes;
-  const uint32_t bar0 = inter + kTileWideBytes;
+  static_assert(!kStaged || kUnits == 1, "one tile per CTA");
+  constexpr TileSmem L = tile_smem(kStaged);
+  const uint32_t inter = slot + L.wide;
+  uint8_t* const interp = smem + L.wide;
+  const uint32_t bar0 = slot + L.bars, bar1 = bar0 + 8;
 
   const int blk0 = 4 * warp;
   int32_t zc[PP][2][2];
@@ -948,6 +963,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
 
   if (tid == 0) {
     mbar_init(bar0, W);
+    if (kStaged) mbar_init(bar1, 1);
     fence_mbar_init();
   }
   __syncthreads();
@@ -1010,8 +1026,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), kb = P.k[b];
     const int j0 = (t - P.first_tile[b]) * tile_jobs(kb, kUnits);
     const int nj = min(tile_jobs(kb, kUnits), P.njobs[b] - j0);
-    bulk_prefetch_l2(P.A[b] + (size_t)j0 * kb * kb * 256, (uint32_t)nj * kb * kb * 512u);
-    if (P.e[b]) bulk_prefetch_l2(P.e[b] + (size_t)j0 * kb * 128, (uint32_t)nj * kb * 512u);
+    const uint32_t na = (uint32_t)nj * kb * kb * 512u, ne = (uint32_t)nj * kb * 512u;
+    if constexpr (kStaged) {
+      mbar_expect_tx(bar1, na + (P.e[b] ? ne : 0));
+      bulk_g2s(slot + L.A, P.A[b] + (size_t)j0 * kb * kb * 256, na, bar1);
+      if (P.e[b]) bulk_g2s(slot + L.e, P.e[b] + (size_t)j0 * kb * 128, ne, bar1);
+      return;
+    }
+    bulk_prefetch_l2(P.A[b] + (size_t)j0 * kb * kb * 256, na);
+    if (P.e[b]) bulk_prefetch_l2(P.e[b] + (size_t)j0 * kb * 128, ne);
   };
 
   // A tile's three phases.  The NTT phases depend on the tile's unit count
@@ -1062,7 +1085,9 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
         for (int i = 0; i < kRows; i++)
 #pragma unroll
           for (int j = 0; j < K; j++)
-            a[i][j] = __ldcs((const uint4*)(Aj + ((i0 + i) * K + j) * 256));
+            a[i][j] = kStaged ? *(const uint4*)(slotp + L.A +
+                                                ((jl * K + i0 + i) * K + j) * 512 + 16 * lane)
+                              : __ldcs((const uint4*)(Aj + ((i0 + i) * K + j) * 256));
       };
       load_a(0);
 #pragma unroll
@@ -1097,9 +1122,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     load_am(g_tile_inv.sb, iam);
     const int32_t cbz[2][4] = {{kCentre, kCentre, kCentre, kCentre},
                                {kCentre, kCentre, kCentre, kCentre}};
-    poly_stage<true, true, kR>(slot + kR * warp * kRowBytes, slotp + kR * warp * kRowBytes, ldt_inv,
-                               iam, 0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + kR * warp, nvec,
-                               8u * g8 + q4);
+    if constexpr (kStaged)  // rows of the tile
+      poly_stage<true, true, kR, true>(
+          slot + kR * warp * kRowBytes, slotp + kR * warp * kRowBytes, ldt_inv, iam, 0, 0, cbz, 0, 0,
+          w_nat, (const uint32_t*)(slotp + L.e), kR * warp,
+          P.e[b] ? min(nvec - row0, tile_rows(P.k[b], kUnits)) : 0, 8u * g8 + q4);
+    else
+      poly_stage<true, true, kR>(slot + kR * warp * kRowBytes, slotp + kR * warp * kRowBytes,
+                                 ldt_inv, iam, 0, 0, cbz, 0, 0, w_nat, P.e[b], row0 + kR * warp,
+                                 nvec, 8u * g8 + q4);
     fence_proxy_async_smem();
     if (NU == W)
       __syncwarp();
@@ -1113,13 +1144,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   using UN = std::integral_constant<int, kUnits>;
 
   issue_load(0);
+  if (kStaged) prefetch(0);
   for (int k = 0; k < nmine; k++) {
-    const bool ok = mbar_wait_bounded(bar0, (uint32_t)k & 1u, kWaitLimitNs);
+    bool ok = mbar_wait_bounded(bar0, (uint32_t)k & 1u, kWaitLimitNs);
     if (!__syncthreads_and(ok)) {  // CTA-uniform give-up
       if (tid == 0) atomicOr(&g_status, 16u);
+      if (kStaged) mbar_wait_bounded(bar1, 0, kWaitLimitNs);  // its own copies in flight
       break;
     }
-    prefetch(k);
+    if (!kStaged) prefetch(k);
     const int t = (int)blockIdx.x + k * G, b = batch_of(t), tl = t - P.first_tile[b];
     const int kb = P.k[b];  // CTA-uniform
     const int row0 = tl * tile_rows(kb, kUnits), nvec = P.njobs[b] * kb;
@@ -1127,7 +1160,15 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
       fwd_phase(U3{});
     else
       fwd_phase(UN{});
-    cta_sync_named();
+    if constexpr (kStaged) {
+      ok = mbar_wait_bounded(bar1, 0, kWaitLimitNs);
+      if (!__syncthreads_and(ok)) {
+        if (tid == 0) atomicOr(&g_status, 16u);
+        break;
+      }
+    } else {
+      cta_sync_named();
+    }
     switch (kb) {
       case 2: basemul_phase(std::integral_constant<int, 2>{}, b, tl); break;
       case 3: basemul_phase(std::integral_constant<int, 3>{}, b, tl); break;
@@ -1295,10 +1336,11 @@ static bool upload_tables_current_device() {
   return cudaMemcpyToSymbol(g_status, &zero, sizeof(zero)) == cudaSuccess;
 }
 
-static const void* tile_fn(int units) {
-  return units == 4   ? (const void*)k_matvec_tiles<4>
-         : units == 2 ? (const void*)k_matvec_tiles<2>
-                      : (const void*)k_matvec_tiles<1>;
+static const void* tile_fn(int units, bool staged) {
+  return staged       ? (const void*)k_matvec_tiles<1, true>
+         : units == 4 ? (const void*)k_matvec_tiles<4, false>
+         : units == 2 ? (const void*)k_matvec_tiles<2, false>
+                      : (const void*)k_matvec_tiles<1, false>;
 }
 
 bool mma_init_device(DeviceInfo* info) {
@@ -1342,13 +1384,16 @@ bool mma_init_device(DeviceInfo* info) {
   }
   {
     info->tile_ctas_per_sm = 1 << 20;
-    for (int units = 4; units >= 1; units >>= 1) {
-      const void* fn = tile_fn(units);
-      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem) !=
+    for (int kind = 0; kind < 4; kind++) {
+      const bool staged = kind == 3;
+      const void* fn = tile_fn(staged ? 1 : 4 >> kind, staged);
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               tile_smem(staged).bytes) !=
           cudaSuccess)
         return false;
       int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, kTileSmem) != cudaSuccess)
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, tile_smem(staged).bytes) !=
+          cudaSuccess)
         return false;
       per_sm = per_sm > 0 ? per_sm : 1;
       if (per_sm < info->tile_ctas_per_sm) info->tile_ctas_per_sm = per_sm;
@@ -1507,7 +1552,7 @@ cudaError_t launch_mma(bool inverse, int variant, const int16_t* src, int16_t* d
 }
 
 cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceInfo& info,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool host_inputs) {
   if (nb > kMaxSegs) return cudaErrorInvalidValue;
   const long long cap = (long long)info.num_sms * info.tile_ctas_per_sm;
   // Tile kind: the smallest tiles that make one round of resident CTAs (592), since
@@ -1534,6 +1579,11 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
                             (!any3 || tiles_of(2) <= two || tiles_of(4) > two)
                         ? 2
                         : 4;
+  // Host memory: staged up to a tile per eight SMs (18).  Beyond, the link's rate decides,
+  // and s waiting behind all of A costs a little.  Plain / staged, us: 24 jobs of k = 4
+  // (12 tiles) 25.1 / 23.9, 37 27.4 / 27.3, 48 29.6 / 29.8, 64 33.1 / 33.9, 128 48.6 /
+  // 50.2, 1,000 267 / 271; 200 of k = 2 (50 tiles) 33.7 / 34.9.
+  const bool staged = host_inputs && units == 1 && tiles_of(1) <= (size_t)info.num_sms / 8;
   MvTiles m = {};
   for (int b = 0; b < nb; b++) {
     const MatvecPart& B = batches[b];
@@ -1557,7 +1607,7 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = (size_t)kTileSmem;
+  cfg.dynamicSmemBytes = (size_t)tile_smem(staged).bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1565,7 +1615,7 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   void* args[1] = {(void*)&m};
-  return cudaLaunchKernelExC(&cfg, tile_fn(units), args);
+  return cudaLaunchKernelExC(&cfg, tile_fn(units, staged), args);
 }
 
 // Self-test of the give-up path: one CTA waits, through the same bounded

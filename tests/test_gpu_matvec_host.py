@@ -43,8 +43,8 @@ def layout(kind, specs):
 
 KINDS = ["packed", "apart", "in_place", "no_addend", "misaligned", "out_is_e", "out_in_A",
          "out_half_over_s", "out_is_next_s", "outs_overlap"]
-SPECS = [((3, 1),), ((4, 37),), ((2, 5), (3, 3), (4, 2)), ((2, 1), (3, 2), (4, 3), (2, 4), (3, 5)),
-         ((3, 700), (2, 9))]
+SPECS = [((3, 1),), ((4, 36),), ((4, 37),), ((2, 5), (3, 3), (4, 2)),
+         ((2, 1), (3, 2), (4, 3), (2, 4), (3, 5)), ((3, 700), (2, 9))]
 
 
 def run(tk, arena, lay, outs=None):
@@ -79,7 +79,7 @@ def test_page_locked_arena_as_pageable(tk, cuda, kind, specs):
 
 @pytest.mark.parametrize("locked_inputs", [True, False])
 def test_one_side_page_locked(tk, cuda, locked_inputs):
-    lay, size = layout("packed", SPECS[2])
+    lay, size = layout("packed", SPECS[3])
     data = rng(5).integers(-32768, 32768, size=size).astype(np.int16)
     want = data.copy()
     run(tk, want, lay)
