@@ -532,6 +532,24 @@ __global__ void __launch_bounds__(
     fence_mbar_init();
   }
   __syncthreads();
+  // The CTA's first tile into L2 while the previous kernel in the stream still drains:
+  // memory idles between the two, and the first loads, which every CTA waits for,
+  // then find their lines near.  Only a prefetch, so it may come before the wait
+  // below: what the previous kernel still writes there goes through the same L2.  From
+  // one and a half tiles per CTA, us: 40,009 polynomials forward 10.1 -> 9.0, inverse
+  // 11.8 -> 10.5, 100,003 20.0 -> 18.7 and 22.5 -> 21.3; 28,000 6.87 -> 6.76 from L2, 7.9 ->
+  // 6.9 from memory.  Below, inputs in L2 lose (16,411 4.71 -> 4.82, a round trip of 20,000
+  // 12.6 -> 13.3) and only inputs in memory gain (16,411 6.2 -> 5.3).  Two tiles ahead:
+  // 40,009 9.9.
+  if constexpr (!kMulti) {
+    if (lane == 0 && 2 * nunits >= 3 * G * W && warp < tile_units_of(0)) {
+      const int row = 8 * (tile_unit0(0) + warp);
+      if constexpr (kSplitIn)
+        tma_prefetch_3d(&segs.in, 0, 0, row);
+      else
+        tma_prefetch_2d(&segs.in, 0, row);
+    }
+  }
   // Everything above overlaps the previous kernel in the stream; from here on
   // global memory that it may have written is read.
   grid_dependency_wait();
@@ -903,11 +921,16 @@ __host__ __device__ constexpr int tile_rows(int k, int units) {
 }
 __host__ __device__ constexpr int tile_jobs(int k, int units) { return tile_rows(k, units) / k; }
 
-// kStaged (one-unit tiles, one per CTA, on host memory): A and e of the tile come into
+// kStagedForm (one-unit tiles, one per CTA, on host memory): A and e of the tile come into
 // shared memory beside s, so that a call waits for the link once, not for s, A and e
 // in turn.  Host to host, us: 1 job of k = 3 18.2 -> 15.7, 5 of k = 4 21.0 -> 17.7, 20 of
 // k = 3 21.4 -> 19.2, 36 of k = 4 27.7 -> 27.1.  On device memory the extra hop costs 0.1 us of 2.8.
-template <int kUnits, bool kStaged>
+// kAheadForm: the first tile's s, A and e into L2 before the wait for the previous
+// kernel in the stream, as the batch kernels.  The rule stands at launch_matvec_tile;
+// built separately because the untaken branch alone cost 6,000 jobs of k = 2 12.5 -> 13.0
+// us.
+enum TileForm { kPlain, kStagedForm, kAheadForm };
+template <int kUnits, TileForm kForm>
 __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__ MvTiles P) {
   constexpr int W = 4, PP = 2;  // PP: block pairs per warp
   extern __shared__ __align__(128) uint8_t smem[];
@@ -921,11 +944,28 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
   const int nmine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / G + 1 : 0;
   const uint32_t slot = smem_u32(smem);
   uint8_t* const slotp = smem;
+  constexpr bool kStaged = kForm == kStagedForm;
   static_assert(!kStaged || kUnits == 1, "one tile per CTA");
   constexpr TileSmem L = tile_smem(kStaged);
   const uint32_t inter = slot + L.wide;
   uint8_t* const interp = smem + L.wide;
   const uint32_t bar0 = slot + L.bars, bar1 = bar0 + 8;
+
+  if (kForm == kAheadForm && lane == 0) {
+    const int t = (int)blockIdx.x;
+    int b = 0;
+#pragma unroll
+    for (int j = 1; j < kMaxSegs; j++) b += (j < P.nb && t >= P.first_tile[j]);
+    const int kb = P.k[b], tl = t - P.first_tile[b];
+    const int row = tl * tile_rows(kb, kUnits) + 8 * warp;
+    if (warp < tile_units(kb, kUnits) && row < P.njobs[b] * kb)
+      tma_prefetch_2d(&P.s_map[b], 0, row);
+    if (warp == 0) {
+      const int j0 = tl * tile_jobs(kb, kUnits), nj = min(tile_jobs(kb, kUnits), P.njobs[b] - j0);
+      bulk_prefetch_l2(P.A[b] + (size_t)j0 * kb * kb * 256, (uint32_t)nj * kb * kb * 512u);
+      if (P.e[b]) bulk_prefetch_l2(P.e[b] + (size_t)j0 * kb * 128, (uint32_t)nj * kb * 512u);
+    }
+  }
 
   const int blk0 = 4 * warp;
   int32_t zc[PP][2][2];
@@ -1336,11 +1376,12 @@ static bool upload_tables_current_device() {
   return cudaMemcpyToSymbol(g_status, &zero, sizeof(zero)) == cudaSuccess;
 }
 
-static const void* tile_fn(int units, bool staged) {
-  return staged       ? (const void*)k_matvec_tiles<1, true>
-         : units == 4 ? (const void*)k_matvec_tiles<4, false>
-         : units == 2 ? (const void*)k_matvec_tiles<2, false>
-                      : (const void*)k_matvec_tiles<1, false>;
+static const void* tile_fn(int units, TileForm form) {
+  return form == kStagedForm  ? (const void*)k_matvec_tiles<1, kStagedForm>
+         : form == kAheadForm ? (const void*)k_matvec_tiles<4, kAheadForm>
+         : units == 4         ? (const void*)k_matvec_tiles<4, kPlain>
+         : units == 2         ? (const void*)k_matvec_tiles<2, kPlain>
+                              : (const void*)k_matvec_tiles<1, kPlain>;
 }
 
 bool mma_init_device(DeviceInfo* info) {
@@ -1384,9 +1425,10 @@ bool mma_init_device(DeviceInfo* info) {
   }
   {
     info->tile_ctas_per_sm = 1 << 20;
-    for (int kind = 0; kind < 4; kind++) {
+    for (int kind = 0; kind < 5; kind++) {
       const bool staged = kind == 3;
-      const void* fn = tile_fn(staged ? 1 : 4 >> kind, staged);
+      const void* fn =
+          kind < 3 ? tile_fn(4 >> kind, kPlain) : tile_fn(0, staged ? kStagedForm : kAheadForm);
       if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                tile_smem(staged).bytes) !=
           cudaSuccess)
@@ -1584,6 +1626,14 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
   // (12 tiles) 25.1 / 23.9, 37 27.4 / 27.3, 48 29.6 / 29.8, 64 33.1 / 33.9, 128 48.6 /
   // 50.2, 1,000 267 / 271; 200 of k = 2 (50 tiles) 33.7 / 34.9.
   const bool staged = host_inputs && units == 1 && tiles_of(1) <= (size_t)info.num_sms / 8;
+  // Ahead from one and a quarter rounds of tiles.  Without / with, us: 30,000 jobs of k =
+  // 2 39.8 / 37.6, 12,000 of k = 3 31.6 / 28.6, 12,000 of k = 4 42.4 / 39.0, 16,383 mixed
+  // 36.7 / 35.5, 65,536 mixed 122 / 120 at full clock; 750 tiles (6,000 of k = 3) 18.9 /
+  // 18.0; 625 tiles 18.4 / 19.0 (k = 2), 15.7 / 15.9 (k = 3), 22.7 / 21.3 (k = 4); one round
+  // (4,095 mixed) 12.9 / 13.3.
+  const TileForm form = staged ? kStagedForm
+                        : units == 4 && 4 * tiles_of(4) >= 5 * (size_t)cap ? kAheadForm
+                                                                           : kPlain;
   MvTiles m = {};
   for (int b = 0; b < nb; b++) {
     const MatvecPart& B = batches[b];
@@ -1615,7 +1665,7 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   void* args[1] = {(void*)&m};
-  return cudaLaunchKernelExC(&cfg, tile_fn(units, staged), args);
+  return cudaLaunchKernelExC(&cfg, tile_fn(units, form), args);
 }
 
 // Self-test of the give-up path: one CTA waits, through the same bounded

@@ -165,6 +165,9 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
   const int nmine = (P.ntiles - 1 - (int)blockIdx.x) / G + 1;
   auto tile_row = [&](int k) { return kPkTile * (k * G + (int)blockIdx.x); };
 
+  // the first tile into L2 ahead of the wait for the previous kernel (only a prefetch):
+  // 100,003 polynomials 2-bit 15.5 -> 14.9 us, 3-bit 16.6 -> 15.4
+  if (warp == kPkLoadWarp && lane == 0) tma_prefetch_2d(&P.in, 0, tile_row(0));
   const uint32_t bars = base + L::kOffBars;
   constexpr int S = L::kInSlots;
   auto in_full = [&](int s) { return bars + 8u * s; };

@@ -144,6 +144,18 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, int c0, int c1, u
       : "memory");
 }
 
+// The box of such a load into L2 only; nothing waits for it.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap),
+               "r"(c0), "r"(c1)
+               : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_3d(const void* tmap, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(tmap),
+               "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+
 // ---- bulk async copies (TMA, non-tensor) -------------------------------------
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes,
                                          uint32_t bar) {
