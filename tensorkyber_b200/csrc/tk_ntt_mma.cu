@@ -87,6 +87,7 @@ __device__ unsigned int g_status;
 struct OneSeg {
   CUtensorMap in;
   CUtensorMap out;
+  const void* src;  // what `in` describes
   const uint32_t* addend;
   int npoly;
 };
@@ -536,15 +537,21 @@ __global__ void __launch_bounds__(
   // memory idles between the two, and the first loads, which every CTA waits for,
   // then find their lines near.  Only a prefetch, so it may come before the wait
   // below: what the previous kernel still writes there goes through the same L2.  From
-  // one and a half tiles per CTA, us: 40,009 polynomials forward 10.1 -> 9.0, inverse
-  // 11.8 -> 10.5, 100,003 20.0 -> 18.7 and 22.5 -> 21.3; 28,000 6.87 -> 6.76 from L2, 7.9 ->
-  // 6.9 from memory.  Below, inputs in L2 lose (16,411 4.71 -> 4.82, a round trip of 20,000
-  // 12.6 -> 13.3) and only inputs in memory gain (16,411 6.2 -> 5.3).  Two tiles ahead:
-  // 40,009 9.9.
+  // one and a half tiles per CTA the tile's TMA boxes, us: 40,009 polynomials forward
+  // 10.1 -> 9.0, inverse 11.8 -> 10.5, 100,003 20.0 -> 18.7 and 22.5 -> 21.3 (two tiles
+  // ahead: 40,009 9.9).  Below, where that costs inputs that are in L2 already (16,411
+  // 4.68 -> 4.82, a round trip of 20,000 12.8 -> 13.3), plain spans, which cost them nothing
+  // (4.64, 12.9): inputs in memory 16,411 6.2 -> 5.3 and 6.9 -> 6.4, 24,000 inverse 8.5 ->
+  // 8.1; with two tiles per CTA those are the slower ones (inverse, 40,009, 10.75).
+  // None with one unit per CTA (1,021: 1.74 -> 1.77).
   if constexpr (!kMulti) {
-    if (lane == 0 && 2 * nunits >= 3 * G * W && warp < tile_units_of(0)) {
+    if (lane == 0 && nunits > G && warp < tile_units_of(0)) {
       const int row = 8 * (tile_unit0(0) + warp);
-      if constexpr (kSplitIn)
+      constexpr int kRow = C::kPackBytes ? C::kPackBytes : 512;
+      if (2 * nunits < 3 * G * W)
+        bulk_prefetch_l2((const uint8_t*)segs.src + (size_t)row * kRow,
+                         (uint32_t)min(8, segs.npoly - row) * kRow);
+      else if constexpr (kSplitIn)
         tma_prefetch_3d(&segs.in, 0, 0, row);
       else
         tma_prefetch_2d(&segs.in, 0, row);
@@ -1503,6 +1510,7 @@ cudaError_t launch_fwd_form(int form, const void* src, int16_t* dst, long long n
                   encode_batch_map(&m.out, dst + done * 256, n);
     if (!ok) return cudaErrorInvalidResourceHandle;
     m.npoly = n;
+    m.src = in;
     const cudaError_t e = launch_variant(V, cap, m, n, stream);
     if (e != cudaSuccess) return e;
   }
@@ -1550,6 +1558,7 @@ cudaError_t launch_mma_segs(bool inverse, int variant, const Seg* segs, int nseg
         return cudaErrorInvalidResourceHandle;
       m.addend = (const uint32_t*)pc[0].addend;
       m.npoly = pc[0].n;
+      m.src = pc[0].src;
       np = 0;
       return launch_variant(V, cap, m, m.npoly, stream);
     }

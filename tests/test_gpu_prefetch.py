@@ -6,8 +6,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# 148 SMs x 3 (forward) or 4 (inverse) CTAs x 32 polynomials x 1.5 tiles: 21,312 and 28,416
-SIZES = [21304, 21305, 21313, 28408, 28409, 28417, 60000, 262145]
+# 148 SMs x 3 (forward) or 4 (inverse) CTAs x 8 polynomials, and x 32 x 1.5 tiles
+SIZES = [3552, 3553, 4736, 4737, 16411, 21304, 21305, 21313, 28408, 28409, 28417, 60000, 262145]
 
 
 def ints(gen, shape, lo, hi, dtype):
