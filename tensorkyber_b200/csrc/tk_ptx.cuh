@@ -323,7 +323,8 @@ __device__ __forceinline__ void tc_ld64_sync(uint32_t taddr, uint32_t (&r)[64]) 
       : "memory");
 }
 // Four runs of 8 consecutive 32-bit columns of this thread's lane (r[8 i ..] from
-// t_i), waited for in the same statement as tc_ld64_sync.
+// t_i), waited for in the same statement as tc_ld64_sync.  The first three loads
+// write their registers before the last one reads its address: early clobber.
 __device__ __forceinline__ void tc_ld8x4_sync(uint32_t t0, uint32_t t1, uint32_t t2, uint32_t t3,
                                               uint32_t (&r)[32]) {
   asm volatile(
@@ -332,11 +333,12 @@ __device__ __forceinline__ void tc_ld8x4_sync(uint32_t t0, uint32_t t1, uint32_t
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%34];\n\t"
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%35];\n\t"
       "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]),
+        "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]),
+        "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(r[16]), "=&r"(r[17]),
+        "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+        "=r"(r[30]), "=r"(r[31])
       : "r"(t0), "r"(t1), "r"(t2), "r"(t3)
       : "memory");
 }
