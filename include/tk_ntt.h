@@ -121,12 +121,14 @@ typedef struct tk_matvec_batch {
 } tk_matvec_batch;
 int tk_matvec(const tk_matvec_batch *batches, int nbatches, tk_stream_t stream);
 /* tk_matvec on HOST buffers, synchronous (the plain per-request launch).
- * Page-locked, device-mapped buffers are used in place: the kernel writes out
- * straight to them, and reads A, s and e there when all of them are page-locked
- * too and no out overlaps any of them (its own s exactly is fine).  What is not
- * goes through a device staging buffer per device that grows to the largest
- * call (at most 8 GiB, also for calls that need none of it), inputs in one copy
- * when they are contiguous, A then s then e.  Calls on one device are
+ * Up to 1 MiB of buffers (A, s, e and out together), page-locked, device-mapped
+ * ones are used in place: the kernel writes out straight to them, and reads A, s
+ * and e there when all of them are page-locked too and no out overlaps any of
+ * them (its own s exactly is fine).  A larger call would keep the kernel on the
+ * GPU, in the way of other streams' kernels, for as long as the link takes.  What
+ * is not used in place goes through a device staging buffer per device that grows
+ * to the largest call (at most 8 GiB, also for calls that need none of it), inputs
+ * in one copy when they are contiguous, A then s then e.  Calls on one device are
  * serialised.  out may alias s. */
 int tk_matvec_host(const tk_matvec_batch *batches, int nbatches);
 /* tk_matvec_host for callers that must not allocate (no counterpart in the
@@ -210,10 +212,13 @@ int tk_server_destroy(tk_server *srv, double timeout_s);
  * transform / copy-out chunk of tk_ntt_host / tk_invntt_host (1 .. 32768, the
  * default; smaller chunks are slower on a B200 host link: the path runs at the
  * link rate).  The first chunks of a call grow from 4096 polynomials to it and
- * the last ones shrink back, so the copies that cannot overlap stay short. */
+ * the last ones shrink back, so the copies that cannot overlap stay short.
+ * TK_OPT_MATVEC_HOST_IN_PLACE (read only): what the calling thread's last
+ * tk_matvec_host used in place: 0 nothing, 1 the outputs, 2 outputs and inputs. */
 #define TK_OPT_MATVEC_CHUNK_POLYS 1
 #define TK_OPT_MATVEC_MODE 2
 #define TK_OPT_HOST_CHUNK_POLYS 3
+#define TK_OPT_MATVEC_HOST_IN_PLACE 4
 #define TK_MATVEC_PIPELINE 0
 #define TK_MATVEC_FUSED 1
 #define TK_MATVEC_TILED 2

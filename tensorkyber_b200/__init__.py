@@ -359,7 +359,7 @@ def matvec_host_noalloc(batches, stream=0):
 
 def matvec_host(batches):
     """tk_matvec on numpy int16 host arrays (synchronous; same shapes as matvec;
-    page-locked arrays are used in place)."""
+    page-locked arrays of up to 1 MiB in all are used in place)."""
     items = []
     for k, A, s, e, out in batches:
         n = _host_arr(s) // k
@@ -441,6 +441,7 @@ class Server:
 # chunk) or MATVEC_FUSED (one kernel, one warp per job).
 OPT_MATVEC_CHUNK_POLYS = 1
 OPT_HOST_CHUNK_POLYS = 3
+OPT_MATVEC_HOST_IN_PLACE = 4  # get_option only: 0, 1 (outputs) or 2 (all), last matvec_host
 OPT_MATVEC_MODE = 2
 MATVEC_PIPELINE, MATVEC_FUSED, MATVEC_TILED = 0, 1, 2
 

@@ -40,6 +40,7 @@ struct DeviceState {
 
 DeviceState g_dev[kMaxDevices];
 thread_local char t_err[256] = "";
+thread_local int t_host_in_place = 0;  // TK_OPT_MATVEC_HOST_IN_PLACE
 
 // Kernel variant choice: forced by tk_set_variant (>= 0) or picked by size.
 std::atomic<int> g_forced[2] = {{-1}, {-1}};
@@ -584,13 +585,15 @@ int tk_matvec(const tk_matvec_batch* batches, int nbatches, tk_stream_t stream) 
 
 // Host buffers that the tile kernel can use where they are: 0 none, 1 every output,
 // 2 every output and every input; dev: the list with those buffers' device addresses.
-// Wanted: page-locked mapped memory, 16-byte aligned, one launch for the list (more
-// batches would be ordered by launch), outputs that overlap no other buffer but
-// their own s exactly (staged inputs are all read before the kernel starts, so with
-// those the outputs need only be apart from each other).
+// Wanted: at most kMatvecInPlaceBytes in all (bytes), page-locked mapped memory,
+// 16-byte aligned, one launch for the list (more batches would be ordered by
+// launch), outputs that overlap no other buffer but their own s exactly (staged
+// inputs are all read before the kernel starts, so with those the outputs need only
+// be apart from each other).
 static int direct_host_buffers(const tk_matvec_batch* batches, int nbatches, int nonempty,
-                               tk_matvec_batch* dev) {
-  if (nonempty > tk::kMaxSegs || g_matvec_mode.load(std::memory_order_relaxed) != TK_MATVEC_TILED)
+                               size_t bytes, tk_matvec_batch* dev) {
+  if (bytes > tk::kMatvecInPlaceBytes || nonempty > tk::kMaxSegs ||
+      g_matvec_mode.load(std::memory_order_relaxed) != TK_MATVEC_TILED)
     return 0;
   auto usable = [](const void* d) { return d && ((uintptr_t)d & 15u) == 0; };
   bool inputs = true;
@@ -626,6 +629,7 @@ static int direct_host_buffers(const tk_matvec_batch* batches, int nbatches, int
 
 int tk_matvec_host(const tk_matvec_batch* batches, int nbatches) {
   t_err[0] = 0;
+  t_host_in_place = 0;
   int nonempty = 0;
   int rc = validate_matvec(batches, nbatches, true, &nonempty);
   if (rc || nonempty == 0) return rc;
@@ -648,12 +652,13 @@ int tk_matvec_host(const tk_matvec_batch* batches, int nbatches) {
   DeviceState& S = g_dev[dev];
   std::lock_guard<std::mutex> lk(S.mv_mu);
   std::vector<tk_matvec_batch> dev_batches((size_t)nbatches);
-  // Page-locked buffers without copies: a copy engine's copy costs 5-8 us before its
-  // first byte, the kernel's own reads and posted writes over the link do not, and
-  // the output leaves while later inputs arrive.  Host to host, copies / outputs in
-  // place / all in place, us: 1 job of k = 3 23.7 / 19.7 / 18.9; 37 of k = 4 37.5 /
-  // 30.2 / 27.7; 1,000 of k = 4 288 / 284 / 265; 4,000 of k = 3 697 / 697 / 648.
-  const int direct = direct_host_buffers(batches, nbatches, nonempty, dev_batches.data());
+  // Small requests in page-locked buffers go without copies: a copy engine's copy
+  // costs 5-8 us before its first byte, the kernel's own reads and posted writes over
+  // the link do not, and the output leaves while later inputs arrive.  Host to host,
+  // copies / outputs in place / all in place, us: 1 job of k = 3 23.7 / 19.7 / 18.9; 37
+  // of k = 4 37.5 / 30.2 / 27.7 (the size limit: kMatvecInPlaceBytes).
+  const int direct = direct_host_buffers(batches, nbatches, nonempty, need, dev_batches.data());
+  t_host_in_place = direct;
   cudaError_t e = cudaSuccess;
   if (!S.mv_stream) e = cudaStreamCreateWithFlags(&S.mv_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess && direct < 2 && S.mv_bytes < need) {
@@ -952,6 +957,7 @@ long long tk_get_option(int option) {
     case TK_OPT_MATVEC_CHUNK_POLYS: return g_matvec_chunk.load();
     case TK_OPT_MATVEC_MODE: return g_matvec_mode.load();
     case TK_OPT_HOST_CHUNK_POLYS: return g_host_chunk.load();
+    case TK_OPT_MATVEC_HOST_IN_PLACE: return t_host_in_place;
     default: return -TK_ERR_INVALID_VALUE;
   }
 }
