@@ -490,11 +490,11 @@ static int validate_matvec(const tk_matvec_batch* batches, int nbatches, bool ho
   return TK_SUCCESS;
 }
 
-// Launches a validated batch list of device buffers.
-static int launch_matvec_batches(const tk_matvec_batch* batches, int nbatches,
+// Launches a validated batch list of device buffers in `mode`, which an entry point
+// reads once (another thread may set it meanwhile).
+static int launch_matvec_batches(const tk_matvec_batch* batches, int nbatches, int mode,
                                  const DeviceInfo* info, cudaStream_t stream,
                                  bool host_inputs = false) {
-  const int mode = g_matvec_mode.load(std::memory_order_relaxed);
   if (mode == TK_MATVEC_TILED) {  // one tile-kernel launch per kMaxSegs batches
     tk::MatvecPart parts[tk::kMaxSegs];
     int np = 0;
@@ -580,7 +580,8 @@ int tk_matvec(const tk_matvec_batch* batches, int nbatches, tk_stream_t stream) 
     for (const void* p : ptrs)
       if (p && (rc = check_device_ptr(p))) return rc;
   }
-  return launch_matvec_batches(batches, nbatches, info, (cudaStream_t)stream);
+  return launch_matvec_batches(batches, nbatches, g_matvec_mode.load(std::memory_order_relaxed),
+                               info, (cudaStream_t)stream);
 }
 
 // Host buffers that the tile kernel can use where they are: 0 none, 1 every output,
@@ -591,9 +592,8 @@ int tk_matvec(const tk_matvec_batch* batches, int nbatches, tk_stream_t stream) 
 // inputs are all read before the kernel starts, so with those the outputs need only
 // be apart from each other).
 static int direct_host_buffers(const tk_matvec_batch* batches, int nbatches, int nonempty,
-                               size_t bytes, tk_matvec_batch* dev) {
-  if (bytes > tk::kMatvecInPlaceBytes || nonempty > tk::kMaxSegs ||
-      g_matvec_mode.load(std::memory_order_relaxed) != TK_MATVEC_TILED)
+                               int mode, size_t bytes, tk_matvec_batch* dev) {
+  if (bytes > tk::kMatvecInPlaceBytes || nonempty > tk::kMaxSegs || mode != TK_MATVEC_TILED)
     return 0;
   auto usable = [](const void* d) { return d && ((uintptr_t)d & 15u) == 0; };
   bool inputs = true;
@@ -657,7 +657,9 @@ int tk_matvec_host(const tk_matvec_batch* batches, int nbatches) {
   // the link do not, and the output leaves while later inputs arrive.  Host to host,
   // copies / outputs in place / all in place, us: 1 job of k = 3 23.7 / 19.7 / 18.9; 37
   // of k = 4 37.5 / 30.2 / 27.7 (the size limit: kMatvecInPlaceBytes).
-  const int direct = direct_host_buffers(batches, nbatches, nonempty, need, dev_batches.data());
+  const int mode = g_matvec_mode.load(std::memory_order_relaxed);
+  const int direct =
+      direct_host_buffers(batches, nbatches, nonempty, mode, need, dev_batches.data());
   t_host_in_place = direct;
   cudaError_t e = cudaSuccess;
   if (!S.mv_stream) e = cudaStreamCreateWithFlags(&S.mv_stream, cudaStreamNonBlocking);
@@ -704,7 +706,7 @@ int tk_matvec_host(const tk_matvec_batch* batches, int nbatches) {
     D.out = direct ? direct_out : dout;
   }
   if (e == cudaSuccess) {
-    rc = launch_matvec_batches(dev_batches.data(), nbatches, info, st, direct == 2);
+    rc = launch_matvec_batches(dev_batches.data(), nbatches, mode, info, st, direct == 2);
     if (rc) {
       cudaStreamSynchronize(st);
       return rc;
@@ -805,7 +807,8 @@ int tk_matvec_host_noalloc(const tk_matvec_batch* batches, int nbatches, tk_stre
     D.out = dout;
   }
   if (e == cudaSuccess) {
-    rc = launch_matvec_batches(dev_batches, nbatches, info, st);
+    rc = launch_matvec_batches(dev_batches, nbatches,
+                               g_matvec_mode.load(std::memory_order_relaxed), info, st);
     if (rc) {
       cudaStreamSynchronize(st);
       return rc;
