@@ -55,6 +55,7 @@
 
 #include "tk_internal.h"
 #include "tk_ptx.cuh"
+#include "tk_split.h"
 #include "tk_stages.cuh"
 #include "tk_tables.h"
 
@@ -445,25 +446,8 @@ __global__ void __launch_bounds__(
     nunits = segs.first_unit[segs.nseg];
   else
     nunits = (segs.npoly + 7) >> 3;
-  // Work split.  Whole tiles are dealt round robin, tile k of CTA c being the
-  // (k G + c)-th of the batch; the units left over, less than a tile per CTA, are
-  // split evenly into a last, short tile each.  So the launch moves through the
-  // batch as one front, upwards in the forward and downwards in the inverse: an
-  // inverse after a forward on the same memory starts on what was written last
-  // and is still in L2 (126 MB): ntt then invntt in place, us in a long loop,
-  // 200,000 polynomials (102 MB) 89.9 -> 83.5, 262,144 100.8 -> 97.5; one run of
-  // units per CTA before.
-  const int G = (int)gridDim.x, cta = (int)blockIdx.x;
-  const int whole = nunits / (G * W);
-  const int left = nunits - whole * G * W;
-  const int left0 = (int)((long long)cta * left / G);
-  const int nlast = (int)((long long)(cta + 1) * left / G) - left0;
-  const int nmine = whole + (nlast > 0);  // tiles of this CTA (CTA-uniform)
-  auto tile_units_of = [&](int k) { return k < whole ? W : nlast; };
-  auto tile_unit0 = [&](int k) {
-    const int i = k < whole ? (k * G + cta) * W : whole * G * W + left0;
-    return kInverse ? nunits - i - tile_units_of(k) : i;
-  };
+  const FrontTiles<W, kInverse> split(nunits, (int)gridDim.x, (int)blockIdx.x);
+  const int nmine = split.tiles();  // CTA-uniform
 
   const uint32_t smem0 = smem_u32(smem);
   const uint32_t inter = smem0 + C::kSlots * C::kSlotBytes;  // wide: int32 intermediates
@@ -545,10 +529,10 @@ __global__ void __launch_bounds__(
   // 8.1; with two tiles per CTA those are the slower ones (inverse, 40,009, 10.75).
   // None with one unit per CTA (1,021: 1.74 -> 1.77).
   if constexpr (!kMulti) {
-    if (lane == 0 && nunits > G && warp < tile_units_of(0)) {
-      const int row = 8 * (tile_unit0(0) + warp);
+    if (lane == 0 && nunits > split.G && warp < split.units(0)) {
+      const int row = 8 * (split.unit0(0) + warp);
       constexpr int kRow = C::kPackBytes ? C::kPackBytes : 512;
-      if (2 * nunits < 3 * G * W)
+      if (2 * nunits < 3 * split.G * W)
         bulk_prefetch_l2((const uint8_t*)segs.src + (size_t)row * kRow,
                          (uint32_t)min(8, segs.npoly - row) * kRow);
       else if constexpr (kSplitIn)
@@ -651,9 +635,9 @@ __global__ void __launch_bounds__(
   };
   auto issue_load = [&](int k, int slot_i) {
     if (lane != 0) return;
-    const int unit = tile_unit0(k) + warp;
+    const int unit = split.unit0(k) + warp;
     const uint32_t bar = bar0 + 8 * slot_i;
-    if (warp < tile_units_of(k)) {
+    if (warp < split.units(k)) {
       const int sg = seg_of(unit);
       const CUtensorMap* tm_in = map_in(sg);
       const int row = 8 * (unit - seg_first(sg));
@@ -674,8 +658,8 @@ __global__ void __launch_bounds__(
   };
   auto issue_store = [&](int k, int slot_i) {
     if (lane != 0) return;
-    const int unit = tile_unit0(k) + warp;
-    if (warp < tile_units_of(k)) {
+    const int unit = split.unit0(k) + warp;
+    if (warp < split.units(k)) {
       const int sg = seg_of(unit);
       tma_store_2d(map_out(sg), 0, 8 * (unit - seg_first(sg)),
                    smem0 + slot_i * C::kSlotBytes + warp * C::kUnitBytes);
@@ -763,7 +747,7 @@ __global__ void __launch_bounds__(
     uint8_t* minep = slotp + 8 * warp * kRowBytes;
 
     if constexpr (kShortTile) {
-      const int nu = tile_units_of(k);  // live units; CTA-uniform
+      const int nu = split.units(k);  // live units; CTA-uniform
       if (nu <= 3 * W / 4) {  // the CTA's last tile
         if (nu <= W / 4)
           short_tile(std::integral_constant<int, W / 4>{}, slot, slotp);
@@ -778,7 +762,7 @@ __global__ void __launch_bounds__(
     if constexpr (kWide && kInverse) {
       block_stage_inv_wide<W>(slot, blk0, ldc_off, interp, ia_row, ia, ac, cc);
       cta_sync_named();
-      const int unit = tile_unit0(k) + warp;
+      const int unit = split.unit0(k) + warp;
       poly_stage_inv_wide<kAdd>(inter + 8 * warp * kWideRowBytes, minep, lb, amw, cb,
                                 w_nat, kAdd ? seg_addend(0) : nullptr, 8 * unit,
                                 kAdd ? seg_npoly(0) : 0, 8u * g8 + q4);
@@ -794,7 +778,7 @@ __global__ void __launch_bounds__(
         poly_stage_small<kIn, true>(mine, irow0, ldt_off,
                                     slotp + C::kRowsBytes + warp * 8 * C::kPackBytes, ab, cb_lo,
                                     cb_hi, wi_e, wi_o, lane, &tile_bad);
-        if (warp < tile_units_of(k)) bad |= tile_bad;
+        if (warp < split.units(k)) bad |= tile_bad;
       }
       cta_sync_named();
       block_stage_wide<W, C::kPairsPerWarp, C::kUnitBytes>(inter, slotp, blk0, ldw, stc_off, ac);
@@ -812,7 +796,7 @@ __global__ void __launch_bounds__(
         poly_stage_small<kIn>(mine, minep, ldt_off,
                               slotp + C::kRowsBytes + warp * 8 * C::kPackBytes, ab, cb_lo, cb_hi,
                               w_even, w_odd, lane, &tile_bad);
-        if (warp < tile_units_of(k)) bad |= tile_bad;
+        if (warp < split.units(k)) bad |= tile_bad;
       }
       cta_sync_named();
       block_stage<true, false, W>(slot, slotp, blk0, ldc_off, stc_off, ac, cc);
@@ -822,7 +806,7 @@ __global__ void __launch_bounds__(
     } else {
       block_stage<false, true, W>(slot, slotp, blk0, ldc_off, stc_off, ac, cc);
       cta_sync_named();
-      const int unit = tile_unit0(k) + warp;
+      const int unit = split.unit0(k) + warp;
       const int sg = kAdd ? seg_of(unit) : 0;
       poly_stage<true, kAdd>(mine, minep, ldt_off, am, cm_lo, cm_hi, cb, 0, 0, w_nat,
                              kAdd ? seg_addend(sg) : nullptr,
@@ -913,21 +897,6 @@ __host__ __device__ constexpr TileSmem tile_smem(bool staged) {
   const int e = A + (staged ? 8 * 4 * 512 : 0), bars = e + (staged ? 8 * 512 : 0);
   return TileSmem{wide, A, e, bars, bars + 16};
 }
-// Tiles of a launch of kind `units` (4, 2 or 1): 8-row shared-memory units, rows of
-// the batch and jobs per tile.  k = 3: 24 rows, the smallest whole number of both
-// jobs and units, or, with units = 1, two jobs in six rows of one unit (six-row
-// TMA boxes).
-__host__ __device__ constexpr int tile_units(int k, int units) {
-  return k == 3 && units > 1 ? 3 : units;
-}
-__host__ __device__ constexpr int tile_box_rows(int k, int units) {
-  return k == 3 && units == 1 ? 6 : 8;
-}
-__host__ __device__ constexpr int tile_rows(int k, int units) {
-  return tile_units(k, units) * tile_box_rows(k, units);
-}
-__host__ __device__ constexpr int tile_jobs(int k, int units) { return tile_rows(k, units) / k; }
-
 // kStagedForm (one-unit tiles, one per CTA, on host memory): A and e of the tile come into
 // shared memory beside s, so that a call waits for the link once, not for s, A and e
 // in turn.  Host to host, us: 1 job of k = 3 18.2 -> 15.7, 5 of k = 4 21.0 -> 17.7, 20 of

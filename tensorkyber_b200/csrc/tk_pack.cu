@@ -60,6 +60,7 @@
 
 #include "tk_internal.h"
 #include "tk_ptx.cuh"
+#include "tk_split.h"
 #include "tk_tables.h"
 #include "tk_umma.cuh"
 
@@ -162,8 +163,10 @@ __global__ void __launch_bounds__(kPkThreads, 1) k_ntt_packed(const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = (int)gridDim.x;
   // tiles round robin: the launch moves through the batch as one front
-  const int nmine = (P.ntiles - 1 - (int)blockIdx.x) / G + 1;
-  auto tile_row = [&](int k) { return kPkTile * (k * G + (int)blockIdx.x); };
+  const int nmine = front_tile_count(P.ntiles, G, (int)blockIdx.x);
+  auto tile_row = [&](int k) {
+    return kPkTile * front_tile(P.ntiles, G, (int)blockIdx.x, k, false);
+  };
 
   // the first tile into L2 ahead of the wait for the previous kernel (only a prefetch):
   // 100,003 polynomials 2-bit 15.5 -> 14.9 us, 3-bit 16.6 -> 15.4

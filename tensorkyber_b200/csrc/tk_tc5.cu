@@ -68,6 +68,7 @@
 
 #include "tk_internal.h"
 #include "tk_ptx.cuh"
+#include "tk_split.h"
 #include "tk_tables.h"
 #include "tk_umma.cuh"
 
@@ -178,10 +179,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc5(const __grid_constant__ T
   // tiles round robin, the whole launch one front through the batch: upwards in
   // the forward, downwards in the inverse, which then starts on what a forward on
   // the same memory wrote last (as the mma.sync kernels)
-  const int nmine = (P.ntiles - 1 - (int)blockIdx.x) / G + 1;
+  const int nmine = front_tile_count(P.ntiles, G, (int)blockIdx.x);
   auto tile_row = [&](int k) {
-    const int t = k * G + (int)blockIdx.x;
-    return kTcTile * (kInverse ? P.ntiles - 1 - t : t);
+    return kTcTile * front_tile(P.ntiles, G, (int)blockIdx.x, k, kInverse);
   };
 
   // the first tile into L2 while the previous kernel in the stream drains (no more than
