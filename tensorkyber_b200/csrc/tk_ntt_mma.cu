@@ -677,6 +677,8 @@ __global__ void __launch_bounds__(
   // 100,003 25.0 -> 23.1.  Unrolled for each size: as loops over units 6,000
   // polynomials took 3.13 instead of 3.01 us (262,144: 48.4).
   constexpr bool kShortTile = !kMulti && !kAdd;
+  // every row of a short tile is live (the range check of kInSmall counts them all)
+  static_assert(kIn != kInSmall || W == 4, "short tiles of exactly their units");
   auto short_tile = [&](auto nc, uint32_t slot, uint8_t* slotp) {
     constexpr int NU = decltype(nc)::value, R = NU * 8 / W;
     const int row = R * warp;  // this warp's first row in the stages over m
