@@ -883,10 +883,10 @@ struct MvTiles {
 
 __device__ int32_t g_tile_z[128];  // basemul pair roots z_t (build_pair_roots)
 // The tiled kernel's inverse: stage A on the basemul's parity-split rows
-// (non-negative: no bias to cancel), stage B scaled by 2^-16, the factor its
-// basemul leaves out (basemul_row_z).
+// (non-negative: no bias to cancel), stage B (InvFrags::sb) scaled by 2^-16, the
+// factor its basemul leaves out (basemul_row_z).
 __device__ TileFrags g_tile_sa;
-__device__ InvFrags g_tile_inv;
+__device__ uint32_t g_tile_sb[2][32][4];
 
 // Shared memory of a CTA: the slot, the forward's int32 sums, in the staged form A
 // (16 KB) and e of the tile, and two mbarriers.
@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(128, 4) k_matvec_tiles(const __grid_constant__
     cta_sync_named();
     constexpr int kR = 2 * NU;  // rows per warp
     uint32_t iam[2][4];
-    load_am(g_tile_inv.sb, iam);
+    load_am(g_tile_sb, iam);
     const int32_t cbz[2][4] = {{kCentre, kCentre, kCentre, kCentre},
                                {kCentre, kCentre, kCentre, kCentre}};
     if constexpr (kStaged)  // rows of the tile
@@ -1345,7 +1345,7 @@ static bool upload_tables_current_device() {
   });
   if (cudaMemcpyToSymbol(g_fwd, &FF, sizeof(FF)) != cudaSuccess) return false;
   if (cudaMemcpyToSymbol(g_inv, &IF, sizeof(IF)) != cudaSuccess) return false;
-  if (cudaMemcpyToSymbol(g_tile_inv, &IFR, sizeof(IFR)) != cudaSuccess) return false;
+  if (cudaMemcpyToSymbol(g_tile_sb, IFR.sb, sizeof(IFR.sb)) != cudaSuccess) return false;
   if (cudaMemcpyToSymbol(g_tile_sa, &TF, sizeof(TF)) != cudaSuccess) return false;
   int32_t z[128];
   build_pair_roots(z);
