@@ -61,9 +61,7 @@ const char* const kVariantNames[tk::kNumMmaVariants] = {
 };
 
 // Autotuned choice per direction and size bucket floor(log2(npoly)); -1 =
-// not tuned: variant 3 for the forward; for the inverse variant 0 below 2^19
-// polynomials and variant 2 from there (the fastest shapes measured at 2^18
-// and 2^20).
+// not tuned (choose_variant).
 constexpr int kBuckets = 33;
 std::atomic<int> g_tuned[2][kBuckets];
 struct TunedInit {
@@ -84,10 +82,13 @@ int choose_variant(bool inverse, size_t npoly) {
   if (f >= 0) return f;
   const int t = g_tuned[inverse ? 1 : 0][size_bucket(npoly)].load(std::memory_order_relaxed);
   if (t >= 0) return t;
-  // untuned: the measured best per direction (forward: the int32-tile
-  // mma.sync kernel everywhere; inverse: the tcgen05 kernel from 2^18
-  // polynomials, where it leads, the 3-slot mma.sync kernel below, where the
-  // tcgen05 kernel's larger CTA costs more to start)
+  // Untuned.  Forward: the int32-tile mma.sync kernel everywhere.  Inverse: the
+  // tcgen05 kernel from 2^18 polynomials, the 3-slot mma.sync kernel below, where
+  // the tcgen05 kernel's larger CTA costs more to start and its 128-polynomial tiles
+  // are dealt whole.  us in a graph, tcgen05 / mma.sync: 20,000 polynomials 9.1 / 6.2,
+  // 100,003 21.7 / 21.5, 262,144 45.0 / 52.0, 2^20 162 / 198.  131,072, one tile short
+  // of seven whole rounds, is already better there (26.9 / 28.5 in a long loop, and
+  // tk_autotune picks it); the line stands above the sizes where the last round decides.
   return inverse ? (npoly >= ((size_t)1 << 18) ? tk::kTc5Variant : 0) : 3;
 }
 
@@ -450,7 +451,7 @@ static bool overlaps(const void* a, size_t na, const void* b, size_t nb) {
 
 // Checks of a batch list common to the device and host forms; *nonempty =
 // batches with work.  host: pointers are host memory (no alignment or overlap
-// rule, the data is staged).
+// rule: what cannot be used where it is is staged).
 static int validate_matvec(const tk_matvec_batch* batches, int nbatches, bool host,
                            int* nonempty_out) {
   if (nbatches < 0 || (nbatches > 0 && !batches)) {

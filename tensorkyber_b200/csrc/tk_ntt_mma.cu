@@ -854,22 +854,16 @@ __global__ void __launch_bounds__(
 // registers hold the basemul's loads in flight.  Every mbarrier wait is
 // bounded (2 s; sets status bit 4 and stops the CTA).
 // Bound by instruction issue and load latency (16 warps per SM at 39 % of
-// the issue slots), not DRAM, so instructions come out wherever an
-// intermediate's form is this kernel's own: ntt(s) reduced lazily, A words
-// multiplied packed (dp2a), the accumulators written parity-split and unbiased
-// for stage A, e added as packed pairs.  65,536 jobs, k ~ U{2,3,4}: 143.8 ->
-// 133.3 us; 1,023 jobs 7.8 -> 7.05 us.  The basemul in place (two slots of 17 KB
-// instead of three, the rest left to L1) and k = 4's A in two halves: 133.3 ->
-// 129.4 us; in a seconds-long loop, where the 1 kW limit holds the clock and
-// energy counts, 140.1 -> 136.2.  A 24-row tile's polynomial stages on all four
-// warps, six rows each, instead of eight on three: k = 3 alone 70.2 -> 66.4 us,
-// the mix 129.6 -> 126.3.  The forward on int32 sums as the batch kernel's variant
-// 3 (20 instructions per polynomial fewer), in the room of the second slot: 125.5
-// -> 121.8 us, 16,383 jobs 36.8 -> 36.0 (in a long loop 39.9 -> 37.5); with both
-// slots kept, three CTAs per SM, 129 us.  Five or six CTAs per SM at 96 or 80
-// registers: 133.2 / 132.6 us.  Smaller tiles in calls that leave CTAs idle: 24
-// jobs of k = 3 5.3 -> 3.0 us, 2,000 of k = 2 6.6 -> 4.9 (the rule stands at
-// launch_matvec_tile).
+// the issue slots), not DRAM, and in a seconds-long loop by the 1 kW limit, so
+// instructions come out wherever an intermediate's form is this kernel's own: the
+// forward on unreduced int32 sums as the batch kernel's variant 3, A words multiplied
+// packed (dp2a), the accumulators written parity-split and unbiased for stage A, e
+// added as packed pairs; and a 24-row tile's polynomial stages run on all four warps,
+// six rows each.  65,536 jobs, k ~ U{2,3,4}: 143.8 us without these, 120-122 with (a
+// call in a long loop 150 / 134).  One slot and four CTAs per SM: two slots beside the sums
+// leave three CTAs, 129; five or six CTAs at 96 or 80 registers 133.  Smaller tiles in
+// calls that leave CTAs idle: 24 jobs of k = 3 5.3 -> 3.0 us, 2,000 of k = 2 6.6 -> 4.9
+// (the rule stands at launch_matvec_tile).
 struct MvTiles {
   CUtensorMap s_map[kMaxSegs];    // s rows [njobs * k][128 words], 8 x 132-word boxes
   CUtensorMap out_map[kMaxSegs];  // out rows, the same shape (may equal s_map: in place)
@@ -1601,10 +1595,10 @@ cudaError_t launch_matvec_tile(const MatvecPart* batches, int nb, const DeviceIn
                             (!any3 || tiles_of(2) <= two || tiles_of(4) > two)
                         ? 2
                         : 4;
-  // Host memory: staged up to a tile per eight SMs (18).  Beyond, the link's rate decides,
-  // and s waiting behind all of A costs a little.  Plain / staged, us: 24 jobs of k = 4
-  // (12 tiles) 25.1 / 23.9, 37 27.4 / 27.3, 48 29.6 / 29.8, 64 33.1 / 33.9, 128 48.6 /
-  // 50.2, 1,000 267 / 271; 200 of k = 2 (50 tiles) 33.7 / 34.9.
+  // Host memory (requests of up to 1 MiB, at most 60 tiles): staged up to a tile per
+  // eight SMs (18).  Beyond, the link's rate decides, and s waiting behind all of A
+  // costs a little.  Plain / staged, us: 24 jobs of k = 4 (12 tiles) 25.1 / 23.9, 37 27.4
+  // / 27.3, 48 29.6 / 29.8, 64 33.1 / 33.9; 200 of k = 2 (50 tiles) 33.7 / 34.9.
   const bool staged = host_inputs && units == 1 && tiles_of(1) <= (size_t)info.num_sms / 8;
   // Ahead from one and a quarter rounds of tiles.  Without / with, us: 30,000 jobs of k =
   // 2 39.8 / 37.6, 12,000 of k = 3 31.6 / 28.6, 12,000 of k = 4 42.4 / 39.0, 16,383 mixed

@@ -17,8 +17,8 @@
 //     the offset of the first form adds nothing; its small bytes toggle less
 //     of the multipliers than sign-extended ones.  |P +- M| < 2^20.
 //   * The operand goes from the packed words straight to tensor memory, a mask, an
-//     exclusive or and a shift per two operand words.  Nothing is staged in shared
-//     memory.
+//     exclusive or and a shift per two operand words: only the packed rows pass
+//     through shared memory.
 //   * One exact reduction per output, in the pair: the quotients are the high
 //     words of S * ceil(2^32 / q) + 2^31 / q (exact floors for either sign in
 //     this range), and S0 + 2^16 S1 - q (q0 + 2^16 q1) is the packed pair, 2.5
@@ -141,7 +141,7 @@ __device__ __forceinline__ void unpack_quarter(const uint4* v, uint32_t (&op)[4]
 }
 
 // S0, S1 (|S| < 2^20) -> the packed pair of their residues in [0, q).  With m
-// = ceil(2^32 / q), S m = S 2^32 / q + S e / q, e = 1976, |S e / q| < 506 k;
+// = ceil(2^32 / q), S m = S 2^32 / q + S e / q, e = 1976, |S e / q| < 623 k;
 // adding 2^31 / q = 645 k keeps the high word at floor(S / q) for S = j q
 // (error from below) and S = j q + q - 1 (2^32 / q = 1290 k from above).
 __device__ __forceinline__ uint32_t reduce_pair(uint32_t s0, uint32_t s1) {

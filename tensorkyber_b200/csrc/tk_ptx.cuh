@@ -242,7 +242,7 @@ __device__ __forceinline__ uint32_t dp2a_hi(uint32_t a, uint32_t b, uint32_t c) 
 }  // namespace tk
 
 // ---- tcgen05 (5th-generation tensor cores, tensor memory) --------------------
-// Used by the TMEM inverse (tk_tc5.cu).  Tensor-memory addresses are
+// Used by tk_tc5.cu and tk_pack.cu.  Tensor-memory addresses are
 // (lane << 16) | column; a warp reaches the 32 lanes 32 * (warp % 4) ...
 namespace tk {
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {

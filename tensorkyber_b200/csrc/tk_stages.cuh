@@ -348,8 +348,9 @@ __device__ __forceinline__ uint4 basemul_row(const uint4 (&a)[K], const uint4 (&
 // tiled kernel's inverse tables carry it) and two products per instruction:
 // dp2a multiplies the two int16 of an A word by two bytes of one ntt(s)
 // operand word, so a pair's A word is never unpacked.  Per pair and j, with
-// b0, b1 = ntt(s_j) in [0, q + 22) and zb = z_t b1 mod q in [0, q + 4)
-// (red_wide of a product below 2^24), the operand words are the bytes
+// b0, b1 = ntt(s_j) in [0, q) (the bounds here hold up to q + 21) and zb = z_t b1
+// mod q in [0, q + 4) (red_wide of a product below 2^24), the operand words are the
+// bytes
 //   w0 = b0.lo, zb.lo, b0.hi, zb.hi     w1 = b1.lo, b0.lo, b1.hi, b0.hi
 // Bound by instructions and load latency: 4 dp2a per pair and j against 4
 // multiply-adds and 2 unpacks, 2 byte permutes per word pair against 3 unpacks.
